@@ -30,6 +30,9 @@ from agama_b200 import workloads
 POTENTIALS = {"triaxial": 1, "disk": 2, "bar": 3, "halo": 4, "galaxy": 5}
 SPHEROID = dict(density=dict(type="Spheroid", mass=1, scaleRadius=1, gamma=1, beta=4, axisRatioZ=0.6),
                 lmax=12, gridSizeR=80, symmetry="axisymmetric")
+# inner slope and axis ratios of the density models (unit mass and scale radius)
+MODELS = {"triaxial": (1.0, (1.0, 0.8, 0.6)), "bar": (0.5, (1.0, 0.7, 0.5)), "halo": (1.0, (1.0, 0.8, 0.6)),
+          "galaxy": (1.0, (1.0, 1.0, 0.6)), "spheroid": (1.0, (1.0, 1.0, 0.6))}
 PATTERN_SPEED = 0.05
 BAR_RADIUS = 5.0                    # orbits of the bar region: starts inside five scale radii
 TARGET_SHELLS, TARGET_STRIPS = 10, 2
@@ -109,19 +112,45 @@ def finder_of(name):
 def particles(name, n, seed):
     """phase-space points (n x 6) of the distribution that goes with the potential"""
     if name == "disk":
-        pot = potential_of(name)
-        return workloads.disk_particles(n, workloads.vcirc_from_force(pot.force), seed=seed)
-    pos = positions(name, n, seed)
-    return workloads.orbit_ics(pos, potential_of(name).potential, seed=seed + 1000003)
+        return workloads.disk_particles(n, disk_vcirc, seed=seed)
+    return workloads.orbit_ics(positions(name, n, seed), model_potential(name), seed=seed + 1000003)
+
+
+# Speeds and times come from the density models behind the potentials and not from the engine, so
+# that the inputs of a seed are the same numbers whatever evaluates the potentials.
+
+def disk_vcirc(R):
+    """circular speed of the Miyamoto-Nagai disk and NFW halo of the disk potential"""
+    disk = 0.1 * R ** 2 / (R ** 2 + 3.3 ** 2) ** 1.5
+    halo = np.log1p(R / 20) / R - 1 / (R + 20)
+    return np.sqrt(disk + halo)
+
+
+def model_potential(name):
+    """positions -> potentials of the ellipsoidal model (of the bulge alone in the galaxy)"""
+    gamma, axes = MODELS[name]
+
+    def potential(x):
+        x = torch.as_tensor(x)
+        if torch.cuda.is_available():
+            x = x.cuda()
+        return torch.cat([dehnen_potential(x[k:k + 20000], gamma, axes) for k in range(0, len(x), 20000)]).cpu().numpy()
+    return potential
+
+
+def circular_period(gamma, E):
+    """of energy E in the spherical model of the same profile (energies below the range: its inner end)"""
+    r = np.logspace(-6, 8, 4001)
+    mass = (r / (1 + r)) ** (3 - gamma)
+    phi = -np.log1p(1 / r) if gamma == 2 else -(1 - (r / (1 + r)) ** (2 - gamma)) / (2 - gamma)
+    return np.exp(np.interp(E, phi + 0.5 * mass / r, np.log(2 * np.pi * np.sqrt(r ** 3 / mass))))
 
 
 def positions(name, n, seed):
-    if name == "bar":
-        return workloads.dehnen_positions(n, 0.5, q=(0.7, 0.5), seed=seed)
     if name == "disk":
         return np.ascontiguousarray(particles(name, n, seed)[:, :3])
-    q = {"triaxial": (0.8, 0.6), "halo": (0.8, 0.6), "galaxy": (1.0, 0.6), "spheroid": (1.0, 0.6)}[name]
-    return workloads.dehnen_positions(n, 1.0, q=q, seed=seed)
+    gamma, axes = MODELS[name]
+    return workloads.dehnen_positions(n, gamma, q=axes[1:], seed=seed)
 
 
 def focal_distances(points, seed):
@@ -134,13 +163,12 @@ def bar_starts(n, seed):
     """starts inside BAR_RADIUS (a fifth of the profile's mass lies outside)"""
     pos = positions("bar", 2 * n + 100, seed)
     pos = pos[np.linalg.norm(pos, axis=1) < BAR_RADIUS][:n]
-    return workloads.orbit_ics(pos, potential_of("bar").potential, seed=seed + 1000003)
+    return workloads.orbit_ics(pos, model_potential("bar"), seed=seed + 1000003)
 
 
 def periods_of(name, ic):
-    pot = potential_of(name)
-    E = pot.potential(ic[:, :3]) + 0.5 * np.sum(ic[:, 3:] ** 2, axis=1)
-    return workloads.tcirc(pot.potential, pot.force, E)
+    E = model_potential(name)(ic[:, :3]) + 0.5 * np.sum(ic[:, 3:] ** 2, axis=1)
+    return circular_period(MODELS[name][0], E)
 
 
 def on_gpu(a):
@@ -253,11 +281,14 @@ def dehnen_rho(m, gamma, axes):
     return (3 - gamma) / (4 * math.pi * axes[1] * axes[2]) * m ** -gamma * (1 + m) ** (gamma - 4)
 
 
-def dehnen_potential(x, axes):
-    """gamma = 1, unit mass and scale radius"""
+def dehnen_potential(x, gamma, axes):
     w, dw, q = ellipsoidal_nodes(x, axes)
     m = w * sum(x[:, i:i + 1] ** 2 / q[i] for i in range(3)).sqrt()
-    return -(dw * (1 + m) ** -2 / (q[0] * q[1] * q[2]).sqrt()).sum(1)
+    u = m / (1 + m)
+    outside = (1 - u ** (2 - gamma)) / (2 - gamma) - (1 - u ** (3 - gamma)) / (3 - gamma)
+    if gamma == 1:
+        outside = 0.5 * (1 + m) ** -2       # the same without its cancellation at large m
+    return -(3 - gamma) * (dw * outside / (q[0] * q[1] * q[2]).sqrt()).sum(1)
 
 
 def dehnen_derivs(x, gamma, axes, hessian):
@@ -289,7 +320,7 @@ def fudge_actions(w, fd, axes):
 
     def phi(lam, nu):
         r2 = ((lam - D) * (1 - nu / D)).clamp(min=0)
-        return dehnen_potential(torch.stack([r2.sqrt(), 0 * r2, (lam * nu / D).clamp(min=0).sqrt()], 1), axes)
+        return dehnen_potential(torch.stack([r2.sqrt(), 0 * r2, (lam * nu / D).clamp(min=0).sqrt()], 1), 1.0, axes)
 
     s = R * R + z * z
     root = ((s - D) ** 2 + 4 * R * R * D).sqrt()
@@ -332,10 +363,9 @@ def fudge_actions(w, fd, axes):
 def exact(case, seed):
     kind, name, n = case["kind"], case["potential"], case["n"]
     device = "cuda" if torch.cuda.is_available() else "cpu"
-    axes = {"triaxial": (1.0, 0.8, 0.6), "bar": (1.0, 0.7, 0.5), "spheroid": (1.0, 1.0, 0.6)}.get(name)
-    if axes is None or kind not in ("force", "hessian", "fixed"):
+    if kind not in ("force", "hessian", "fixed") or name not in ("triaxial", "bar", "spheroid"):
         return None         # sums of models, tables and orbits have no such value
-    gamma = 0.5 if name == "bar" else 1.0
+    gamma, axes = MODELS[name]
     state = prepare(case, seed)
     x = state["points"].to(device)
     parts = []
@@ -344,9 +374,9 @@ def exact(case, seed):
         if kind == "fixed":
             parts.append((fudge_actions(b, state["fd"].to(device)[k:k + 20000], axes),))
         elif kind == "force":
-            parts.append((dehnen_potential(b, axes) if gamma == 1 else None, dehnen_derivs(b, gamma, axes, False)[0]))
+            parts.append((dehnen_potential(b, gamma, axes), dehnen_derivs(b, gamma, axes, False)[0]))
         else:
             m = sum((b[:, i] / axes[i]) ** 2 for i in range(3)).sqrt()
             parts.append(dehnen_derivs(b, gamma, axes, True) + (dehnen_rho(m, gamma, axes),))
-    out = tuple(None if p[0] is None else torch.cat(p) for p in zip(*parts))
+    out = tuple(torch.cat(p) for p in zip(*parts))
     return out[0] if kind == "fixed" else out
