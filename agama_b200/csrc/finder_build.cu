@@ -31,12 +31,15 @@ __global__ void equatorialKernel(const __grid_constant__ MultipoleView M, int n,
     out[4 * i] = Phi; out[4 * i + 1] = g.dR; out[4 * i + 2] = h.dR2; out[4 * i + 3] = h.dz2;
 }
 
-/// focal distance at each (E_i, Lz/Lcirc = L_j) node from its shell orbit
+/** Focal distance at each (E_i, Lz/Lcirc = L_j) node from its shell orbit, one node per block of one
+    thread.  A node is a serial chain (nested root searches over orbits of the meridional system) and
+    its branches have nothing in common with the next node's: 32 nodes in the lanes of one warp ran
+    one after the other (6.3 lanes active), while the ~1700 warps of one lane each leave 3 chains per
+    scheduler to hide each other's latency. */
 __global__ void shellGridKernel(const __grid_constant__ MultipoleView M, int nE, int nL, const double* gridE,
     const double* gridL, double* delta, double* rshell)
 {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if(k >= nE * nL) return;
+    const int k = blockIdx.x;
     const int iE = k / nL, iL = k % nL;
     const double E = gridE[iE];
     const double Rc = shellRcirc(M, E);
@@ -231,7 +234,7 @@ FinderTablesHost buildFinderTables(const DevicePotential& P)
     DevBuf<double> dE, dL, dD(nNodes), dRs(nNodes);
     dE.upload(gridE);
     dL.upload(gridL);
-    shellGridKernel<<<(nNodes + 31) / 32, 32>>>(P.view, nE - 1, nL - 1, dE.ptr, dL.ptr, dD.ptr, dRs.ptr);
+    shellGridKernel<<<nNodes, 1>>>(P.view, nE - 1, nL - 1, dE.ptr, dL.ptr, dD.ptr, dRs.ptr);
     AGB_CUDA(cudaGetLastError());
     std::vector<double> D(nNodes);
     AGB_CUDA(cudaMemcpy(D.data(), dD.ptr, nNodes * sizeof(double), cudaMemcpyDeviceToHost));
