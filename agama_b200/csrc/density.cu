@@ -7,7 +7,7 @@
 // asymptotic expansions give it in closed form (PowerLawMultipole::densityCyl,
 // src/potential_multipole.cpp:1660-1687).
 #include "runtime.h"
-#include "multipole_eval.cuh"
+#include "multipole_cells.cuh"
 
 namespace agb {
 
@@ -61,7 +61,7 @@ __device__ double powerLawDensity(const PowerLawView& A, double R, double z, dou
 }
 
 /// gradient and Hessian of the interpolated potential inside the grid (the interpolator alone,
-/// as the reference's impl object)
+/// as the reference's impl object) from the node form of the splines
 template<int KIND>
 __device__ __forceinline__ void interiorDerivs(const MultipoleView& M, double R, double z, double phi,
     CylDerivs* g, CylHess* h)
@@ -75,34 +75,59 @@ __device__ __forceinline__ void interiorDerivs(const MultipoleView& M, double R,
         evalInterp1d<6>(M, R, z, phi, &Phi, g, h);
 }
 
-/// Laplacian / (4 pi) in cylindrical coordinates with the reference's treatment of the z axis
-/// and of results dominated by round-off (BasePotential::densityCyl)
-template<int KIND>
-__device__ double laplacianDensity(const MultipoleView& M, double R, double z, double phi)
+/// the Laplacian's terms dPhi/dR / R and d2Phi/dphi2 / R^2 added up with the rest of it, and the
+/// treatment of results dominated by round-off (BasePotential::densityCyl)
+__device__ __forceinline__ double densityOfDerivs(const CylHess& h, double dRoverR, double d2phiOverR2)
 {
-    CylDerivs g; CylHess h;
-    interiorDerivs<KIND>(M, R, z, phi, &g, &h);
-    double dRoverR = g.dR / R;
-    double d2phiOverR2 = h.dphi2 / pow2(R);
-    if(R <= fabs(z) * SQRT_DBL_EPS) {        // on or next to the z axis
-        dRoverR = h.dR2;
-        if((M.ind.sym & SYM_ZROT) == SYM_ZROT)
-            d2phiOverR2 = 0;
-        else {                               // d2Phi/dphi2 from a point just off the axis
-            const double Roff = fabs(z) * SQRT_DBL_EPS;
-            CylDerivs go; CylHess ho;
-            interiorDerivs<KIND>(M, Roff, z, phi, &go, &ho);
-            d2phiOverR2 = ho.dphi2 / pow2(Roff);
-        }
-    }
     const double result = h.dR2 + dRoverR + h.dz2 + d2phiOverR2;
     if(!(fabs(result) > EPSREL_DENSITY_DER * (fabs(h.dR2) + fabs(dRoverR) + fabs(h.dz2) + fabs(d2phiOverR2))))
         return 0;
     return result / (4 * M_PI);
 }
 
+/// the density with the reference's treatment of the z axis, from the node form: on or next to the
+/// axis the azimuthal term comes from the potential ~1e-8 of the radius away from it, where the
+/// result carries the rounding of the spline evaluation (up to 1e-2 of the density), and the
+/// reference's own arithmetic is what the result agrees with
 template<int KIND>
-__global__ void __launch_bounds__(DENSITY_BLOCK) densityKernel(const __grid_constant__ MultipoleView M, long n,
+__device__ __noinline__ double axisDensity(const MultipoleView& M, double R, double z, double phi)
+{
+    CylDerivs g; CylHess h;
+    interiorDerivs<KIND>(M, R, z, phi, &g, &h);
+    double d2phiOverR2 = 0;
+    if((M.ind.sym & SYM_ZROT) != SYM_ZROT) {     // d2Phi/dphi2 from a point just off the axis
+        const double Roff = fabs(z) * SQRT_DBL_EPS;
+        CylDerivs go; CylHess ho;
+        interiorDerivs<KIND>(M, Roff, z, phi, &go, &ho);
+        d2phiOverR2 = ho.dphi2 / pow2(Roff);
+    }
+    return densityOfDerivs(h, h.dR2, d2phiOverR2);
+}
+
+/// the rare interiors without cells (lmax <= 2, many harmonics) away from the axis
+template<int KIND>
+__device__ __noinline__ double nodeDensity(const MultipoleView& M, double R, double z, double phi)
+{
+    CylDerivs g; CylHess h;
+    interiorDerivs<KIND>(M, R, z, phi, &g, &h);
+    return densityOfDerivs(h, g.dR / R, h.dphi2 / pow2(R));
+}
+
+/// Laplacian / (4 pi) in cylindrical coordinates (BasePotential::densityCyl)
+template<int KIND>
+__device__ __forceinline__ double laplacianDensity(const MultipoleView& M, double R, double z, double phi)
+{
+    if(R <= fabs(z) * SQRT_DBL_EPS) return axisDensity<KIND>(M, R, z, phi);
+    if(KIND == EVAL_GENERAL || !M.cells) return nodeDensity<KIND>(M, R, z, phi);
+    double Phi, sphi = 0, cphi = 1;
+    if(KIND == EVAL_FAST) sincos(phi, &sphi, &cphi);
+    CylDerivs g; CylHess h;
+    evalCells<6, KIND == EVAL_GENERAL ? EVAL_AXI : KIND>(M, R, z, cphi, sphi, &Phi, &g, &h);
+    return densityOfDerivs(h, g.dR / R, h.dphi2 / pow2(R));
+}
+
+template<int KIND>
+__global__ void __launch_bounds__(DENSITY_BLOCK, 4) densityKernel(const __grid_constant__ MultipoleView M, long n,
     const double* __restrict__ pos, double* __restrict__ rho)
 {
     const long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;

@@ -42,6 +42,24 @@ struct PowerLawView {
     const double* W;      // amplitudes of (r/r0)^v
 };
 
+/** device view of one grid of the 2-D splines, for the search of the cell that holds a value: cell
+    k < n - 1 is (node k, 1 / (node k+1 - node k)) and entry n - 1 the last node, so that two
+    neighbouring 16-byte loads give both nodes of a cell and its reciprocal width.  lut[b] is the
+    last cell that begins at or before the left edge of bin b of an even division of the grid into
+    nlut bins; the bins are at most half as wide as the narrowest cell (up to GRID_LUT_MAX of them),
+    so the search almost never goes beyond the next cell. */
+struct alignas(16) GridNode { double x, invH; };
+struct GridView {
+    const GridNode* cell;
+    const unsigned short* lut;
+    double x0, xEnd, lutScale;      // first and last node, nlut / (xEnd - x0)
+    int n, nlut;
+};
+constexpr int GRID_LUT_MAX = 4096;
+
+/// number of coefficients of one cell of a 2-D spline in monomial form
+constexpr int CELL_COEFS = 36;
+
 /// device view of a complete Multipole potential
 struct MultipoleView {
     HarmIndices ind;
@@ -54,6 +72,11 @@ struct MultipoleView {
     double lnrScale, tauScale;   // (n - 1) / (grid[n-1] - grid[0]): binSearchScaled's first guess
     int splSlot[2 * LMAX_MAX + 1];  // slot of the 2-D spline for m (index m+mmax), -1 if empty
     const double* spl2d;  // [slot][nr][nt][NODE_STRIDE]: f fx fy fxx fxy fyy fxxy fxyy fxxyy pad
+    GridView gridR, gridTau;     // the two grids of the 2-D splines (ln r and tau)
+    /// the 2-D splines cell by cell, [slot][nr-1][nt-1][CELL_COEFS]: the coefficients c_ij of
+    /// s^i t^j (j fastest) with s, t the position in the cell in units of its widths, from the
+    /// lower ln r node and from the tau node nearer the pole; null where there are none (nFast = 0)
+    const double* cells;
     const float* spl2d32; // the same table rounded to FP32 (mixed-precision evaluation of m != 0)
     const double* spl1d;  // [c][nr][3]: f f' f''  (1-D case; all (lmax+1)^2 coefficients)
     int logScaling;

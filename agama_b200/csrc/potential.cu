@@ -1,16 +1,21 @@
 // Multipole potential on the device: table upload and the batched evaluation kernel.
 #include "runtime.h"
-#include "multipole_eval.cuh"
+#include "multipole_cells.cuh"
+#include <algorithm>
 
 namespace agb {
 
 namespace {
 thread_local std::string g_error;
 
-/// One point per thread; 256 threads per block.  NQ = 1 (potential), 3 (+gradient), 6 (+Hessian);
-/// KIND = spline evaluator matching the potential (EvalKind).
+/// One point per thread; 128 threads per block.  NQ = 1 (potential), 3 (+gradient), 6 (+Hessian);
+/// KIND = spline evaluator matching the potential (EvalKind).  Bound by the L1: each lane reads its own
+/// cells, nine 32-byte loads a harmonic at one data-stage cycle per lane (60 % of its rate at 2e6
+/// points of the triaxial lmax 6 potential, value and gradient: 543 us from the node form at 168
+/// registers, 410 from the cells with 16-byte loads at 80 registers, 330 with 32-byte loads; with
+/// the Hessian and the density at 4e5 points 294 -> 174 us).
 template<int NQ, int KIND>
-__global__ void __launch_bounds__(128) evalPotentialKernel(const MultipoleView M, long n,
+__global__ void __launch_bounds__(128, NQ == 6 ? 4 : 6) evalPotentialKernel(const __grid_constant__ MultipoleView M, long n,
     const double* __restrict__ pos, double* __restrict__ phi, double* __restrict__ grad,
     double* __restrict__ hess)
 {
@@ -18,7 +23,7 @@ __global__ void __launch_bounds__(128) evalPotentialKernel(const MultipoleView M
     if(i >= n) return;
     const double x = pos[3 * i], y = pos[3 * i + 1], z = pos[3 * i + 2];
     double p, g[3], h[6];
-    evalMultipoleCar<NQ, KIND>(M, x, y, z, &p, g, h);
+    evalCellsCar<NQ, KIND>(M, x, y, z, &p, g, h);
     if(phi) phi[i] = p;
     if(NQ >= 3 && grad) { grad[3 * i] = g[0]; grad[3 * i + 1] = g[1]; grad[3 * i + 2] = g[2]; }
     if(NQ == 6 && hess)
@@ -30,7 +35,7 @@ __global__ void __launch_bounds__(128) evalPotentialKernel(const MultipoleView M
 /// reference's BasePotentialCyl::evalCyl returns them (no round trip through Cartesian
 /// derivatives, which loses the phi derivatives to cancellation at large R)
 template<int NQ, int KIND>
-__global__ void __launch_bounds__(128) evalPotentialCylKernel(const MultipoleView M, long n,
+__global__ void __launch_bounds__(128, NQ == 6 ? 4 : 6) evalPotentialCylKernel(const __grid_constant__ MultipoleView M, long n,
     const double* __restrict__ pos, double* __restrict__ phi, double* __restrict__ grad,
     double* __restrict__ hess)
 {
@@ -38,13 +43,66 @@ __global__ void __launch_bounds__(128) evalPotentialCylKernel(const MultipoleVie
     if(i >= n) return;
     double p;
     CylDerivs g; CylHess h;
-    evalMultipoleCyl<NQ, KIND>(M, pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], &p, &g, &h);
+    evalCellsCyl<NQ, KIND>(M, pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], &p, &g, &h);
     if(phi) phi[i] = p;
     if(NQ >= 3 && grad) { grad[3 * i] = g.dR; grad[3 * i + 1] = g.dz; grad[3 * i + 2] = g.dphi; }
     if(NQ == 6 && hess) {
         hess[6 * i] = h.dR2; hess[6 * i + 1] = h.dz2; hess[6 * i + 2] = h.dphi2;
         hess[6 * i + 3] = h.dRdz; hess[6 * i + 4] = h.dzdphi; hess[6 * i + 5] = h.dRdphi;
     }
+}
+
+/** The coefficients of the 2-D splines cell by cell (MultipoleView::cells) from the node values: one
+    cell per thread.  Both directions take the Hermite data (value, first and second derivative in
+    units of the cell width) of the two ends to the six monomial coefficients; the values are taken
+    relative to one corner, as the node form does, so that c_00 alone carries the offset.  Cells of
+    the upper half of the tau grid are expanded about their upper node (cellAnchor): towards either
+    pole the m != 0 harmonics vanish with a power of the distance from it, which only an expansion
+    about the pole's own node gives without cancellation (and gives exactly 0 on the axis). */
+__global__ void cellCoefsKernel(int numSlots, int nr, int nt, const GridNode* __restrict__ gr,
+    const GridNode* __restrict__ gt, const double* __restrict__ nodes, double* __restrict__ cells)
+{
+    const long k = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
+    const long perSlot = static_cast<long>(nr - 1) * (nt - 1);
+    if(k >= numSlots * perSlot) return;
+    const int slot = static_cast<int>(k / perSlot), rem = static_cast<int>(k % perSlot);
+    const int xi = rem / (nt - 1), yi = rem % (nt - 1);
+    const double hx = gr[xi + 1].x - gr[xi].x, hy = gt[yi + 1].x - gt[yi].x;
+    auto hermite = [](double v0, double g0, double s0, double v1, double g1, double s1, double* c, int stride) {
+        const double A = v1 - v0 - g0 - 0.5 * s0, B = g1 - g0 - s0, C = s1 - s0;
+        c[0] = v0;
+        c[stride] = g0;
+        c[2 * stride] = 0.5 * s0;
+        c[3 * stride] = 10 * A - 4 * B + 0.5 * C;
+        c[4 * stride] = -15 * A + 7 * B - C;
+        c[5 * stride] = 6 * A - 3 * B + 0.5 * C;
+    };
+    // node layout: 0 f, 1 fx, 2 fy, 3 fxx, 4 fxy, 5 fyy, 6 fxxy, 7 fxyy, 8 fxxyy
+    const int val[3] = { 0, 1, 3 }, dy[3] = { 2, 4, 6 }, dyy[3] = { 5, 7, 8 };
+    const double* ll = nodes + ((static_cast<size_t>(slot) * nr + xi) * nt + yi) * NODE_STRIDE;
+    const double off = cellAnchor(gt[yi].x, gt[yi + 1].x) != gt[yi].x ? ll[NODE_STRIDE] : ll[0];
+    double G[2][3][6];       // [x node][x derivative][power of t]
+    const bool upper = cellAnchor(gt[yi].x, gt[yi + 1].x) != gt[yi].x;
+    const double w = upper ? -hy : hy;      // from the anchor to the other end
+    for(int a = 0; a < 2; a++) {
+        const double* lo = ll + a * static_cast<size_t>(nt) * NODE_STRIDE;
+        const double* up = lo + NODE_STRIDE;
+        const double* base = upper ? up : lo;
+        const double* other = upper ? lo : up;
+        double sx = 1;
+        for(int p = 0; p < 3; p++) {
+            const double o = p == 0 ? off : 0;
+            hermite((base[val[p]] - o) * sx, base[dy[p]] * w * sx, base[dyy[p]] * w * w * sx,
+                    (other[val[p]] - o) * sx, other[dy[p]] * w * sx, other[dyy[p]] * w * w * sx, G[a][p], 1);
+            if(upper)       // powers of the distance below the upper node -> powers of t in [-1, 0]
+                for(int j = 1; j < 6; j += 2) G[a][p][j] = -G[a][p][j];
+            sx *= hx;
+        }
+    }
+    double* c = cells + k * CELL_COEFS;
+    for(int j = 0; j < 6; j++)
+        hermite(G[0][0][j], G[0][1][j], G[0][2][j], G[1][0][j], G[1][1][j], G[1][2][j], c + j, 6);
+    c[0] += off;
 }
 }  // namespace
 
@@ -63,8 +121,6 @@ void launchEvalPotential(const MultipoleView& M, long n, const double* pos, doub
     double* grad, double* hess, cudaStream_t stream, bool cylindrical)
 {
     if(n <= 0) return;
-    // 128 threads (up to 168 registers, no spills for the multi-harmonic kind): 16 % faster than
-    // blocks of 256 at 128 registers with spills (config 1 forces 0.055 against 0.065 ms)
     const int block = 128;
     const long grid = (n + block - 1) / block;
     const int nq = hess ? 6 : grad ? 3 : 1, kind = evalKindOf(M);
@@ -144,6 +200,53 @@ DevicePotential* createDevicePotential(const std::vector<double>& radii,
             }
         }
         for(int s = V.nFast; s < FAST_MAX_HARMONICS; s++) { V.fastM[s] = 0; V.fastSlot[s] = 0; }
+        if(H.is2d) {
+            auto gridView = [](const std::vector<double>& g, DevBuf<GridNode>& cell, DevBuf<unsigned short>& lut) {
+                const int n = static_cast<int>(g.size());
+                std::vector<GridNode> c(n);
+                double narrowest = INFINITY;
+                for(int k = 0; k < n; k++) {
+                    c[k].x = g[k];
+                    c[k].invH = k + 1 < n ? 1 / (g[k + 1] - g[k]) : 0;
+                    if(k + 1 < n) narrowest = std::min(narrowest, g[k + 1] - g[k]);
+                }
+                GridView v;
+                v.n = n;
+                v.x0 = g.front();
+                v.xEnd = g.back();
+                const double bins = 2 * (v.xEnd - v.x0) / narrowest;
+                v.nlut = bins < GRID_LUT_MAX ? std::max(1, static_cast<int>(bins) + 1) : GRID_LUT_MAX;
+                v.lutScale = v.nlut / (v.xEnd - v.x0);
+                // the edge is moved down by a millionth of a bin: a value just below it may be put
+                // into this bin by the rounding of (x - x0) * lutScale
+                std::vector<unsigned short> l(v.nlut);
+                for(int b = 0, k = 0; b < v.nlut; b++) {
+                    const double edge = v.x0 + (b - 1e-6) / v.lutScale;
+                    while(k < n - 2 && g[k + 1] <= edge) k++;
+                    l[b] = static_cast<unsigned short>(k);
+                }
+                cell.upload(c);
+                lut.upload(l);
+                v.cell = cell.ptr;
+                v.lut = lut.ptr;
+                return v;
+            };
+            if(H.lnr.size() < 2 || H.tau.size() < 2 || H.lnr.size() > 65535 || H.tau.size() > 65535)
+                throw std::invalid_argument("Multipole: the grids need between 2 and 65535 nodes");
+            V.gridR = gridView(H.lnr, P->gridCellR, P->gridLutR);
+            V.gridTau = gridView(H.tau, P->gridCellTau, P->gridLutTau);
+            // squares of radii outside the range of normal numbers stay with the node form
+            if(V.nFast > 0 && V.rInnerSq > 1e-280 && V.rOuterSq < 1e280) {
+                const long count = static_cast<long>(H.numSlots) * (V.nr - 1) * (V.nt - 1);
+                P->cells.alloc(count * CELL_COEFS);
+                cellCoefsKernel<<<(count + 127) / 128, 128>>>(H.numSlots, V.nr, V.nt, V.gridR.cell, V.gridTau.cell,
+                    V.spl2d, P->cells.ptr);
+                AGB_CUDA(cudaGetLastError());
+                AGB_CUDA(cudaStreamSynchronize(nullptr));
+            }
+        } else
+            V.gridR = V.gridTau = GridView{};
+        V.cells = P->cells.ptr;
     } catch(...) {
         delete P;
         throw;

@@ -47,6 +47,9 @@ struct DevicePotential {
     int device = 0;
     MultipoleHost host;
     DevBuf<double> lnr, tau, lnrInvH, tauInvH, spl2d, spl1d, innerS, innerU, innerW, outerS, outerU, outerW;
+    DevBuf<GridNode> gridCellR, gridCellTau;
+    DevBuf<double> cells;
+    DevBuf<unsigned short> gridLutR, gridLutTau;
     DevBuf<float> spl2d32;
     MultipoleView view;
     /// the axisymmetric (m = 0) part, used by the action finder (same as the full potential
