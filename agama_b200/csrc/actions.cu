@@ -18,7 +18,7 @@ namespace {
 
 /// Gauss-Legendre rules on [0,1] for the orders 1..20, 25, 32, 40 (the set the reference
 /// tabulates, src/math_glquadrature.h), computed by Newton iteration in extended precision
-struct GLRulesHost { int offset[GL_MAX_ORDER + 1]; std::vector<double> nodes, weights; };
+struct GLRulesHost { int offset[GL_MAX_ORDER + 1]; std::vector<double> nodes, weights, cubic; };
 
 GLRulesHost makeGLRules()
 {
@@ -46,13 +46,17 @@ GLRulesHost makeGLRules()
             x[i] = (1 - t) / 2;                    // ascending nodes on [0, 1]
             w[i] = 1 / ((1 - t * t) * dp * dp);    // = (2 / ((1-t^2) P'^2)) / 2
         }
+        for(int i = 0; i < n; i++) {        // the cubic stretch u = s^2 (3 - 2 s) and its weight
+            g.cubic.push_back(static_cast<double>(x[i] * x[i] * (3 - 2 * x[i])));
+            g.cubic.push_back(static_cast<double>(w[i] * 6 * x[i] * (1 - x[i])));
+        }
         for(int i = 0; i < n; i++) { g.nodes.push_back(static_cast<double>(x[i])); g.weights.push_back(static_cast<double>(w[i])); }
     }
     return g;
 }
 
 /// per-device copy of the quadrature rules (uploaded on first use)
-struct GLDevice { DevBuf<double> nodes, weights; GLRules view; };
+struct GLDevice { DevBuf<double> nodes, weights, cubic; GLRules view; };
 std::mutex g_glMutex;
 std::map<int, GLDevice*> g_gl;
 
@@ -67,9 +71,11 @@ const GLRules& glRulesForCurrentDevice()
     GLDevice* d = new GLDevice;
     d->nodes.upload(host.nodes);
     d->weights.upload(host.weights);
+    d->cubic.upload(host.cubic);
     for(int n = 0; n <= GL_MAX_ORDER; n++) d->view.offset[n] = host.offset[n];
     d->view.nodes = d->nodes.ptr;
     d->view.weights = d->weights.ptr;
+    d->view.cubic = d->cubic.ptr;
     g_gl[dev] = d;
     return d->view;
 }
@@ -81,44 +87,33 @@ constexpr long POINTS_PER_PASS = 1L << 20;     // records of one pass: 128 MB of
 /// from the finder's table; otherwise fd[i], or fd0 if fd is null), integrals of motion, the
 /// limits that need no root search and the brackets of those that do -> one record per point.
 /// Jphi (and NaN Jr, Jz of points without actions) are written directly.  Optional outputs:
-/// Delta used, root-finder iterations (zeroed here, counted by phase 2).  ends[i]: F and F' at the
+/// root-finder iterations (zeroed here, counted by phase 2), inputs of the bracket predictor.  ends[i]: F and F' at the
 /// ends of the record's plain root brackets, for the root searches.
 template<bool FINDER>
 __global__ void __launch_bounds__(PREPARE_BLOCK, 5) fudgePrepareKernel(const __grid_constant__ MultipoleView M,
     const __grid_constant__ FudgeTables F, long n, const double* __restrict__ posvel, const double* __restrict__ fd,
-    double fd0, FudgeRecord* __restrict__ rec, double* __restrict__ act, double* __restrict__ fdOut,
-    int* __restrict__ iters, float* __restrict__ features, FudgeEnds* __restrict__ ends)
+    double fd0, FudgeRecord* __restrict__ rec, double* __restrict__ act, int* __restrict__ iters,
+    float* __restrict__ features, FudgeEnds* __restrict__ ends)
 {
     const long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
     if(i >= n) return;
     double w[6], pc[6];
     for(int c = 0; c < 6; c++) w[c] = posvel[6 * i + c];
     carToCylPosVel(w, pc);
-    double Phi;
-    CylDerivs g; CylHess h;
-    evalMultipoleCylCall<1, EVAL_AXI>(M, pc[0], pc[1], 0, &Phi, &g, &h);   // axisymmetric: no azimuth
+    CellPoint p;
+    p.locate(M, pc[0], pc[1]);
+    const double Phi = p.Phi;
     const double delta = FINDER ? finderFocalDistance(F, pc, Phi) : (fd ? fd[i] : fd0);
     FudgeRecord r;
     double a[3];
     FudgeEnds e;
-    fudgePrepare(M, pc, Phi, delta, r, a, &e);
+    fudgePrepare(M, pc, p, delta, r, a, &e);
     rec[i] = r;
     if(r.valid) ends[i] = e;
     act[3 * i + 2] = a[2];
     if(!r.valid) { act[3 * i] = a[0]; act[3 * i + 1] = a[1]; }
-    if(fdOut) fdOut[i] = delta;
     if(iters) iters[i] = 0;
-    if(features) {
-        // inputs of the bracket predictor: the point's (R, z, vR, vz, vphi) with E and Lz in
-        // scale-free form -- ln r, |z| / r, velocities over the escape speed sqrt(-2 Phi) (so
-        // that E = Phi (1 - v^2 / v_esc^2) and Lz = R vphi follow), ln(Delta / r); symmetric
-        // under z -> -z and Lz -> -Lz like the limits themselves
-        const double r = fmax(sqrt(pc[0] * pc[0] + pc[1] * pc[1]), 1e-300), vesc = sqrt(fmax(-2 * Phi, 1e-300));
-        const float f[6] = { static_cast<float>(log(r)), static_cast<float>(fabs(pc[1]) / r),
-            static_cast<float>(pc[3] / vesc), static_cast<float>((pc[1] >= 0 ? pc[4] : -pc[4]) / vesc),
-            static_cast<float>(fabs(pc[5]) / vesc), static_cast<float>(log(fmax(delta, 1e-300) / r)) };
-        for(int k = 0; k < 6; k++) features[6 * i + k] = f[k];
-    }
+    if(features) bracketFeatures(pc, Phi, delta, features + 6 * i);
 }
 
 /// Optional timing of the phases: while on, every pass records CUDA events on its stream before
@@ -183,14 +178,21 @@ void runActions(const MultipoleView& M, const FudgeTables& F, long n, const doub
         int* it = iters ? iters + first : nullptr;
         double* a = act ? act + 3 * first : actTmp;
         float* f = samples ? samples->features + 6 * first : feat;
-        fudgePrepareKernel<FINDER><<<(count + PREPARE_BLOCK - 1) / PREPARE_BLOCK, PREPARE_BLOCK, 0, stream>>>(
-            M, F, count, posvel + 6 * first, fd ? fd + first : nullptr, fd0, rec, a,
-            fdOut ? fdOut + first : nullptr, it, f, ends);
-        AGB_CUDA(cudaGetLastError());
+        // the focal distance handed to the caller is that of the calls with angles (same bits), so
+        // that passing it back gives the same angles
+        double* fdo = fdOut ? fdOut + first : nullptr;
+        const double* fdi = fd ? fd + first : nullptr;
+        if(angles || fdOut)
+            launchNodePrepare(FINDER, M, F, count, posvel + 6 * first, fdi, fd0, rec, a, fdo, it, f, ends, stream);
+        else {
+            fudgePrepareKernel<FINDER><<<(count + PREPARE_BLOCK - 1) / PREPARE_BLOCK, PREPARE_BLOCK, 0, stream>>>(
+                M, F, count, posvel + 6 * first, fdi, fd0, rec, a, it, f, ends);
+            AGB_CUDA(cudaGetLastError());
+        }
         mark(1);
         if(predict) bp->net->predict(count, feat, pred, stream);
         mark(2);
-        launchFudgeRoots(M, count, rec, ends, it, counter, pred, widths, bp ? bp->stats : nullptr, stream);
+        launchFudgeRoots(M, count, rec, ends, it, counter, pred, widths, bp ? bp->stats : nullptr, angles, stream);
         mark(3);
         if(samples)
             launchBracketTargets(count, rec, samples->target + 3 * first, samples->mask + 3 * first, stream);

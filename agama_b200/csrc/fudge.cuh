@@ -7,7 +7,7 @@
 // ActionFinderAxisymFudge::eval (:954-979); prolate spheroidal coordinates from src/coord.cpp
 // (:266-338, :525-531); L_circ(E) from potential::Interpolator (src/potential_utils.cpp:872-980).
 #pragma once
-#include "multipole_eval.cuh"
+#include "multipole_cells.cuh"
 #include "fudge_types.h"
 
 namespace agb {
@@ -40,7 +40,7 @@ __device__ __forceinline__ void spline1d(const Spline1dView& S, double x, double
 }
 
 /// potential::Interpolator::evalDeriv (src/potential_utils.cpp:872-911): Phi(R), dPhi/dR, d2Phi/dR2
-static __device__ void interpPhi(const FudgeTables& F, double R, double* val, double* der, double* der2)
+static __device__ __forceinline__ void interpPhi(const FudgeTables& F, double R, double* val, double* der, double* der2)
 {
     const double logR = log(R);
     if(logR > ldg(F.PhiofR.t + F.PhiofR.n - 1) && F.coefOut != 0) {
@@ -60,7 +60,7 @@ static __device__ void interpPhi(const FudgeTables& F, double R, double* val, do
 }
 
 /// potential::Interpolator::L_circ (src/potential_utils.cpp:954-980)
-static __device__ double interpLcirc(const FudgeTables& F, double E)
+static __device__ __forceinline__ double interpLcirc(const FudgeTables& F, double E)
 {
     if(!(E >= 1. / F.iInvPhi0 && E <= 0))
         return NAN;
@@ -82,7 +82,7 @@ static __device__ double interpLcirc(const FudgeTables& F, double E)
 }
 
 /// bilinear Delta(xi, chi) (LinearInterpolator2d::evalDeriv, src/math_spline.cpp:2152-2190)
-static __device__ double deltaLookup(const FudgeTables& F, double x, double y)
+static __device__ __forceinline__ double deltaLookup(const FudgeTables& F, double x, double y)
 {
     const int nx = F.nE, ny = F.nL;
     const int xi = binSearch(x, F.gridE, nx), yi = binSearch(y, F.gridL, ny);
@@ -96,73 +96,120 @@ static __device__ double deltaLookup(const FudgeTables& F, double x, double y)
     return T * (U * zll + u * zlu) + t * (U * zul + u * zuu);
 }
 
-/// the fudge's auxiliary function F(tau) and the integrals of motion of one point
-struct FudgeFunction {
-    const MultipoleView* M;
-    double lambda, nu, phi, D2;     // point in prolate spheroidal coordinates (Delta^2 = D2)
-    double E, Lz, I3, flambda, fnu;
-    double Ilam, Inu, L2h;          // I3 - fnu, I3 - flambda and Lz^2 / 2, formed once (derive())
-    int bad;                        // set when a coordinate conversion is invalid
+/** The fudge's auxiliary function F(tau) along one of the two coordinates of a point (the other one
+    stays at its value there); AxisymFunctionFudge::evalDeriv, src/actions_staeckel.cpp:202-252, with
+    prolate spheroidal -> cylindrical coordinates from src/coord.cpp:266-291.
 
-    /// the terms of F that do not depend on tau, from the integrals of motion (the same
-    /// operations as in F itself, so the same bits)
-    __device__ void derive() { Ilam = I3 - fnu; Inu = I3 - flambda; L2h = Lz * Lz / 2; }
+    What does not depend on tau is formed once: with (lambda, nu) the point and D2 = Delta^2,
 
-    /// F(tau) and optionally F', F'' (src/actions_staeckel.cpp:202-252); INL: the potential
-    /// evaluation inlined at this call site instead of the shared out-of-line copy
-    template<bool DER, bool DER2, bool INL = false>
-    __device__ void eval(double tau, double* val, double* der, double* der2) const
+        lambda branch (tau = lambda > D2):  R = c1 sqrt(tau - D2),  z = c2 sqrt(tau),
+                                            r^2 = (tau - D2) + nu
+        nu branch     (tau = nu < D2):      R = c1 sqrt(D2 - tau),  z = c2 sqrt(tau),
+                                            r^2 = tau + (lambda - D2)
+
+    and the derivative along the branch needs no gradient in (R, z): with x = ln r and the latitude
+    psi (tau_spline = tan(psi / 2)), dx/dtau = 1 / (2 r^2) and dpsi/dtau = K / (2 r^2 sqrt(|tau - D2| tau)),
+    K = -sqrt(nu (D2 - nu)) or +sqrt(lambda (lambda - D2)), i.e. -+ D2 c1 c2, with the reciprocal
+    roots that R and z are formed from.  One evaluation takes three reciprocal square roots, one
+    reciprocal, a logarithm and an exponential beside the cell (before: three square roots and five
+    to seven divisions, and the gradient's transformation). */
+struct FudgeBranch {
+    double E, I, L2h, D2;       // I: I3 - fnu (lambda branch) or I3 - flambda; L2h = Lz^2 / 2
+    double mo, ro, c1, c2;      // tau - mo multiplies Phi; r^2 = (tau - D2 or tau) + ro
+    bool lam;
+
+    /// the branch's constants from the point's record (nu enters by its absolute value)
+    __device__ void set(bool lambdaBranch, double lambda, double nu, double D2_, double E_, double Lz, double I3,
+        double flambda, double fnu)
     {
-        double lam, n, mult, I;
-        if(tau >= D2) { lam = tau; n = fabs(nu); mult = lam - n; I = Ilam; }
-        else          { lam = lambda; n = tau; mult = n - lam; I = Inu; }
-        // prolate spheroidal -> cylindrical (src/coord.cpp:266-291)
-        const double absnu = fabs(n), sgn = n >= 0 ? 1 : -1;
-        const double lmd = lam - D2, nmd = absnu - D2;
-        if(nmd > 0 || lmd < 0) {
-            *val = NAN; if(DER) *der = NAN; if(DER2) *der2 = NAN;
-            return;
-        }
-        const double R = sqrt(lmd * (1 - absnu / D2));
-        const double z = sqrt(lam * absnu / D2) * sgn;
-        double Phi;
-        CylDerivs g; CylHess h;
-        // the inlined F, F' of the root searches: the cell evaluated in halves (fewer registers
-        // beside the searches' state, the same bits)
-        if(INL)      evalMultipoleCyl<DER2 ? 6 : DER ? 3 : 1, EVAL_AXI, 1, false, DER && !DER2>(*M, R, z, phi, &Phi, &g, &h);
-        else if(DER2) evalMultipoleCylCall<6, EVAL_AXI>(*M, R, z, phi, &Phi, &g, &h);
-        else if(DER) evalMultipoleCylCall<3, EVAL_AXI>(*M, R, z, phi, &Phi, &g, &h);
-        else         evalMultipoleCylCall<1, EVAL_AXI>(*M, R, z, phi, &Phi, &g, &h);
+        lam = lambdaBranch;
+        E = E_; D2 = D2_; L2h = Lz * Lz / 2;
+        I = lam ? I3 - fnu : I3 - flambda;
+        const double n = fabs(nu), lmd = lambda - D2, inv = 1 / D2;
+        mo = lam ? n : lambda;
+        ro = lam ? n : lmd;
+        c1 = sqrt(lam ? 1 - n * inv : lmd * inv);
+        c2 = sqrt((lam ? n : lambda) * inv);
+    }
+
+    /// F(tau), and with DER its derivative
+    template<bool DER>
+    __device__ __forceinline__ void eval(const MultipoleView& M, double tau, double* val, double* der) const
+    {
         const double tmd = tau - D2;
-        *val = (tmd != 0 ? (E * tau - I - Phi * mult) * tmd : 0) - L2h * tau;
-        if(DER || DER2) {
-            // dR/dtau, dz/dtau along the coordinate that tau moves (lambda or nu): only that pair
-            // is divided out
-            const bool lbranch = tau >= D2;
-            double dRdt, dzdt;
-            if(lbranch) { dRdt = 0.5 * R / lmd; dzdt = 0.5 * z / lam; }
-            else        { dRdt = 0.5 * R / nmd * sgn; dzdt = 0.5 * z / n; }
-            const double dPhidtau = g.dR * dRdt + g.dz * dzdt;
-            if(DER)
-                *der = E * (tau + tmd) - L2h - I - (mult + tmd) * Phi -
-                       (tmd != 0 ? tmd * mult * dPhidtau : 0);
-            if(DER2) {
-                double d2;
-                if(lbranch) {
-                    const double d2Rdl2 = -0.25 * R / pow2(lmd), d2zdl2 = -0.25 * z / pow2(lam);
-                    d2 = h.dR2 * pow2(dRdt) + h.dz2 * pow2(dzdt) + 2 * h.dRdz * dRdt * dzdt +
-                         g.dR * d2Rdl2 + g.dz * d2zdl2;
-                } else {
-                    const double d2Rdn2 = -0.25 * R / pow2(nmd), d2zdn2 = -0.25 * z / pow2(n);
-                    d2 = h.dR2 * pow2(dRdt) + h.dz2 * pow2(dzdt) + 2 * h.dRdz * dRdt * dzdt +
-                         g.dR * d2Rdn2 + g.dz * d2zdn2;
-                }
-                *der2 = 2 * (E - Phi - (mult + tmd) * dPhidtau) - tmd * mult * d2;
+        const double u = fmax(lam ? tmd : -tmd, 0.), rsq = (lam ? tmd : tau) + ro;
+        // zeros are kept out of the reciprocal roots: u -> 0 and tau -> 0 give R = 0 and z = 0
+        const double iu = rsqrtNormal(fmax(u, 1e-280)), it = rsqrtNormal(fmax(tau, 1e-280));
+        const double R = c1 * (u * iu), z = c2 * (tau * it);
+        double Phi, px = 0, ppsi = 0, r2inv;        // Phi, dPhi/dln r, dPhi/dpsi
+        if(inCells(M, rsq)) {
+            const double rinv = rsqrtNormal(rsq), logr = 0.5 * log(rsq);
+            const double y = fmin(z * rcpNormal(fma(rsq, rinv, R)), 1.);
+            r2inv = rinv * rinv;
+            double xl, xh, xi, yl, yh, yi;
+            const int ix = gridCell(M.gridR, logr, &xl, &xh, &xi), iy = gridCell(M.gridTau, y, &yl, &yh, &yi);
+            double P, dummy;
+            cellPolynomial<DER ? 3 : 1>(M.cells + (static_cast<size_t>(ix) * (M.nt - 1) + iy) * CELL_COEFS,
+                (logr - xl) * xi, (y - cellAnchor(yl, yh)) * yi, &P, &px, &ppsi, &dummy, &dummy, &dummy);
+            if(DER) { px *= xi; ppsi *= yi * fma(0.5 * y, y, 0.5); }
+            Phi = P;
+            if(M.logScaling) {
+                const double ex = exp(P);
+                Phi = rcpNormal(M.invPhi0 - ex);
+                if(DER) { const double d = Phi * Phi * ex; px *= d; ppsi *= d; }
             }
+        } else {
+            CylDerivs g; CylHess h;
+            evalBeyondCells<DER ? 3 : 1>(M, R, z, 0, &Phi, &g, &h);
+            r2inv = 1 / rsq;
+            if(DER) { px = R * g.dR + z * g.dz; ppsi = R * g.dz - z * g.dR; }
+        }
+        const double mult = tau - mo;
+        *val = (E * tau - I - Phi * mult) * tmd - L2h * tau;
+        if(DER) {
+            const double K = D2 * (c1 * c2);
+            const double dPhi = 0.5 * r2inv * (px + (lam ? -K : K) * (ppsi * iu * it));
+            *der = E * (tau + tmd) - L2h - I - (mult + tmd) * Phi - (tmd != 0 ? tmd * mult * dPhi : 0);
         }
     }
-    __device__ double value(double tau) const { double v; eval<false, false, true>(tau, &v, nullptr, nullptr); return v; }
+    __device__ __forceinline__ double value(const MultipoleView& M, double tau) const
+    {
+        double v;
+        eval<false>(M, tau, &v, nullptr);
+        return v;
+    }
 };
+
+/// F, F' and F'' on the lambda branch from the potential, its gradient and Hessian at (R, z >= 0)
+__device__ __forceinline__ void fudgeSecond(double E, double I, double L2h, double D2, double mo, double tau, double R,
+    double z, double Phi, const CylDerivs& g, const CylHess& h, double* val, double* der, double* der2)
+{
+    const double tmd = tau - D2, mult = tau - mo;
+    const double dRdt = 0.5 * R / tmd, dzdt = 0.5 * z / tau;
+    const double dPhi = g.dR * dRdt + g.dz * dzdt;
+    const double d2 = h.dR2 * pow2(dRdt) + h.dz2 * pow2(dzdt) + 2 * h.dRdz * dRdt * dzdt -
+        0.25 * (g.dR * R / pow2(tmd) + g.dz * z / pow2(tau));
+    *val = (tmd != 0 ? (E * tau - I - Phi * mult) * tmd : 0) - L2h * tau;
+    *der = E * (tau + tmd) - L2h - I - (mult + tmd) * Phi - (tmd != 0 ? tmd * mult * dPhi : 0);
+    *der2 = 2 * (E - Phi - (mult + tmd) * dPhi) - tmd * mult * d2;
+}
+
+/// the same at any tau of the lambda branch, evaluating the potential there (rare: out of line)
+static __device__ __noinline__ void fudgeSecondAt(const MultipoleView& M, const FudgeBranch& f, double tau,
+    double* val, double* der, double* der2)
+{
+    const double R = f.c1 * sqrt(fmax(tau - f.D2, 0.)), z = f.c2 * sqrt(tau);
+    double Phi;
+    CylDerivs g; CylHess h;
+    evalCellsCyl<6, EVAL_AXI>(M, R, z, 0, &Phi, &g, &h);
+    fudgeSecond(f.E, f.I, f.L2h, f.D2, f.mo, tau, R, z, Phi, g, h, val, der, der2);
+}
+
+/// F(tau) out of line, for the rare single values of phase 1 and the angles
+static __device__ __noinline__ double fudgeValueAt(const MultipoleView& M, const FudgeBranch& f, double tau)
+{
+    return f.value(M, tau);
+}
 
 /// State of one point between the phases of the action computation: the point in prolate
 /// spheroidal coordinates, its integrals of motion, the integration limits known so far and the
@@ -191,102 +238,168 @@ enum { ROOT_NU_MAX = 1, ROOT_LAMBDA_MIN = 2, ROOT_LAMBDA_MAX = 4 };
 /// nu_max bracket); NaN where not evaluated
 struct FudgeEnds { double fPos, dfPos, fD2, dfD2, fNu, dfNu; };
 
-/** The root functions of the three integration limits behind one evaluation site (kind
-    ROOT_NU_MAX, ROOT_LAMBDA_MIN: F(tau) and F'(tau); ROOT_LAMBDA_MAX: F(tau)/tau^2 on
+/** The root functions of the three integration limits behind one evaluation site: F(tau) and F'(tau)
+    for nu_max and lambda_min; with semiInf (lambda_max) F(tau)/tau^2 on
     [u0, inf) mapped to s in [0, 1] by the semi-infinite scaling, AxisymScaledForRootfinder inside
     ScaledFnc<ScalingSemiInf>, src/actions_staeckel.cpp:329-354, src/math_core.h:214-232). */
-__device__ __forceinline__ void limitRootEval(const FudgeFunction& f, int kind, double u0, double x,
-    double* v, double* d)
+__device__ __forceinline__ void limitRootEval(const MultipoleView& M, const FudgeBranch& f, bool semiInf, double u0,
+    double x, double* v, double* d)
 {
-    const bool semiInf = kind == ROOT_LAMBDA_MAX;
     double duds = 1, tau = x;
-    if(semiInf) tau = unscaleSemiInf(u0, x, &duds);
-    const bool far = semiInf && tau > 1e100;
+    if(semiInf) {       // unscaleSemiInf with one reciprocal (x = 1 gives NaN: far)
+        const double w = rcpNormal(1 - x);
+        tau = u0 * exp(x * w);
+        duds = tau * w * w;
+    }
+    const bool far = semiInf && !(tau <= 1e100);
     double fval = 0, fder = 0;
-    if(!far) f.eval<true, false, true>(tau, &fval, &fder, nullptr);
+    if(!far) f.eval<true>(M, tau, &fval, &fder);
     if(!semiInf) { *v = fval; *d = fder; }
     else if(far) { *v = f.E; *d = NAN; }
     else {
-        *v = fval / pow2(tau);
-        *d = (fder - 2 * fval / tau) / pow2(tau) * duds;
+        const double it = rcpNormal(tau), it2 = it * it;
+        *v = fval * it2;
+        *d = (fder - 2 * fval * it) * it2 * duds;
     }
 }
 
-/** The point's F(tau) from its record.  The azimuth given to the potential is 0: the fudge takes
-    only axisymmetric potentials, whose coefficients (and so the index sets of their splines and
-    asymptotes) have m = 0 alone, and their evaluators never read the azimuth; a constant leaves
-    the register free for the searches (the record keeps the point's azimuth for the angles). */
-__device__ __forceinline__ void loadFudgeFunction(const MultipoleView& M, const FudgeRecord& r, FudgeFunction& f)
+/// the branch of a record along which one of its limits is searched or one of its actions integrated
+__device__ __forceinline__ void loadFudgeBranch(const FudgeRecord& r, bool lambdaBranch, FudgeBranch& f)
 {
-    f.M = &M;
-    f.lambda = r.lambda; f.nu = r.nu; f.phi = 0; f.D2 = r.D2;
-    f.E = r.E; f.Lz = r.Lz; f.I3 = r.I3; f.flambda = r.flambda; f.fnu = r.fnu;
-    f.derive();
-    f.bad = 0;
+    f.set(lambdaBranch, r.lambda, r.nu, r.D2, r.E, r.Lz, r.I3, r.flambda, r.fnu);
 }
+
+/// out-of-line value of the potential in the equatorial plane or on the axis at squared radius rsq
+static __device__ __noinline__ double potentialOnAxes(const MultipoleView& M, double rsq, int axis)
+{
+    double Phi;
+    if(inCells(M, rsq)) {
+        const double logr = 0.5 * log(rsq);
+        double xl, xh, xi, yl, yh, yi, dummy;
+        const int ix = gridCell(M.gridR, logr, &xl, &xh, &xi), iy = gridCell(M.gridTau, axis, &yl, &yh, &yi);
+        cellPolynomial<1>(M.cells + (static_cast<size_t>(ix) * (M.nt - 1) + iy) * CELL_COEFS, (logr - xl) * xi,
+            (axis - cellAnchor(yl, yh)) * yi, &Phi, &dummy, &dummy, &dummy, &dummy, &dummy);
+        if(M.logScaling) Phi = rcpNormal(M.invPhi0 - exp(Phi));
+    } else {
+        const double r = sqrt(rsq);
+        CylDerivs g; CylHess h;
+        evalBeyondCells<1>(M, axis ? 0 : r, axis ? r : 0, 0, &Phi, &g, &h);
+    }
+    return Phi;
+}
+
+/** What phase 1 needs of the potential, from the cells: one evaluation with the Hessian at the point
+    (R, |z|) gives F of both branches there up to F'', the value at (lambda, nu = 0) gives the
+    integrals of motion and F(0), and the value on the axis F' at Delta^2.  (The node form evaluates
+    the potential six times.)  The same struct is the evaluator of fudgeLimitsSetup. */
+struct CellPoint {
+    double R, z, Phi, Phi0;
+    CylDerivs g;
+    CylHess h;
+    const MultipoleView* view;
+    const FudgeRecord* rec;
+    __device__ __noinline__ void locate(const MultipoleView& M, double R_, double z_)
+    {
+        view = &M;
+        R = R_; z = fabs(z_);
+        evalCellsCyl<6, EVAL_AXI>(M, R, z, 0, &Phi, &g, &h);           // axisymmetric: no azimuth
+    }
+    __device__ double equatorial(const MultipoleView& M, double rsq) { return Phi0 = potentialOnAxes(M, rsq, 0); }
+    __device__ FudgeBranch branch(bool lambdaBranch) const
+    {
+        FudgeBranch f;
+        loadFudgeBranch(*rec, lambdaBranch, f);
+        return f;
+    }
+    // F(0): the potential at (lambda, nu = 0)
+    __device__ double zero() const { return ((rec->I3 - rec->flambda) - Phi0 * rec->lambda) * rec->D2; }
+    __device__ void second(double* v, double* d, double* d2) const
+    {
+        fudgeSecond(rec->E, rec->I3 - rec->fnu, rec->Lz * rec->Lz / 2, rec->D2, fabs(rec->nu), rec->lambda, R, z, Phi,
+            g, h, v, d, d2);
+    }
+    __device__ void secondAt(double tau, double* v, double* d, double* d2) const
+    {
+        fudgeSecondAt(*view, branch(true), tau, v, d, d2);
+    }
+    __device__ double nuValue(double tau) const { return fudgeValueAt(*view, branch(false), tau); }
+    __device__ double lambdaValue(double tau) const { return fudgeValueAt(*view, branch(true), tau); }
+    // at Delta^2, on the axis (R = 0, z = sqrt(nu)): F needs no potential, F' its value alone
+    __device__ void endD2(double* v, double* d) const
+    {
+        const double n = fabs(rec->nu), D2 = rec->D2, L2h = rec->Lz * rec->Lz / 2;
+        *v = -L2h * D2;
+        *d = rec->E * D2 - L2h - (rec->I3 - rec->fnu) - (D2 - n) * potentialOnAxes(*view, n, 1);
+    }
+    // at |nu|, on the nu branch: the point itself
+    __device__ void endNu(double* v, double* d) const
+    {
+        const double n = fabs(rec->nu), tmd = n - rec->D2, mult = n - rec->lambda, L2h = rec->Lz * rec->Lz / 2;
+        const double I = rec->I3 - rec->flambda, dPhi = 0.5 * (g.dR * R / tmd + g.dz * z / n);
+        *v = (tmd != 0 ? (rec->E * n - I - Phi * mult) * tmd : 0) - L2h * n;
+        *d = rec->E * (n + tmd) - L2h - I - (mult + tmd) * Phi - (tmd != 0 ? tmd * mult * dPhi : 0);
+    }
+};
 
 /** Integration limits of the lambda and nu motions (findIntegrationLimitsAxisym,
     src/actions_staeckel.cpp:360-483), part 1: every decision up to the three root searches, whose
     brackets go into the record; limits that need no root are stored directly (NaN otherwise).
-    ends (may be null) receives F and F' at the ends of the plain brackets (FudgeEnds), which the
-    root searches then take instead of evaluating them: at lambda_pos from the evaluation above,
-    at Delta^2 and |nu| from the same evaluation of F as the searches would make. */
-static __device__ void fudgeLimitsSetup(const FudgeFunction& fnc, FudgeRecord& rec, FudgeEnds* ends = nullptr)
+    ends receives F and F' at the ends of the plain brackets (FudgeEnds), which the
+    root searches then take instead of evaluating them. */
+static __device__ __forceinline__ void fudgeLimitsSetup(const CellPoint& fnc, FudgeRecord& rec, FudgeEnds* ends)
 {
-    const double delta = fnc.D2;
-    const double f_zero = fnc.value(0);
+    const double delta = rec.D2, lambda = rec.lambda;
+    const double f_zero = fnc.zero();
     double f_lambda, df_lambda, d2f_lambda;
-    fnc.eval<true, true>(fnc.lambda, &f_lambda, &df_lambda, &d2f_lambda);
+    fnc.second(&f_lambda, &df_lambda, &d2f_lambda);
     double nu_max = NAN, lambda_min = NAN, lambda_max = NAN;
     double nu_upper = delta, lambda_lower = delta;
     int roots = 0;
-    if(fnc.Lz == 0) {
+    if(rec.Lz == 0) {
         const double dminus = delta * (1 - 1e-15), dplus = delta * (1 + 1e-15);
-        if(fnc.value(dminus) < 0) {
+        if(fnc.nuValue(dminus) < 0) {
             if(f_zero > 0) nu_upper = dminus;
             else nu_max = 0;
         } else
             nu_max = delta;
-        if(fnc.value(dplus) < 0) lambda_lower = dplus;
+        if(fnc.lambdaValue(dplus) < 0) lambda_lower = dplus;
         else lambda_min = delta;
     }
     if(!isFinite(nu_max)) {
         if(f_zero > 0) roots |= ROOT_NU_MAX;           // falls back to |nu| if no root is found
-        else nu_max = fabs(fnc.nu);
+        else nu_max = fabs(rec.nu);
     }
-    double lambda_pos = fnc.lambda, f_pos = f_lambda, df_pos = df_lambda;
+    double lambda_pos = lambda, f_pos = f_lambda, df_pos = df_lambda;
     const double dxToRoot = -f_lambda / df_lambda;
-    if(f_lambda <= 0 || fabs(dxToRoot) < fnc.lambda * FUDGE_MINIMUM_RANGE) {
-        if(df_lambda >= 0) lambda_min = fnc.lambda;
+    if(f_lambda <= 0 || fabs(dxToRoot) < lambda * FUDGE_MINIMUM_RANGE) {
+        if(df_lambda >= 0) lambda_min = lambda;
         if(df_lambda <= 0) {
-            lambda_max = fnc.lambda;
-            if(fnc.lambda == delta) lambda_min = delta;
+            lambda_max = lambda;
+            if(lambda == delta) lambda_min = delta;
         }
         bool nearShell = d2f_lambda < 0 &&
-            pow2(df_lambda) - 2 * f_lambda * d2f_lambda - pow2(fnc.lambda * FUDGE_MINIMUM_RANGE * d2f_lambda) < 0;
-        const double safeOffset = fmin(0.5 * fabs(df_lambda / d2f_lambda), fnc.lambda * FUDGE_MINIMUM_RANGE);
+            pow2(df_lambda) - 2 * f_lambda * d2f_lambda - pow2(lambda * FUDGE_MINIMUM_RANGE * d2f_lambda) < 0;
+        const double safeOffset = fmin(0.5 * fabs(df_lambda / d2f_lambda), lambda * FUDGE_MINIMUM_RANGE);
         lambda_pos += fmax(dxToRoot, safeOffset) * (df_lambda >= 0 ? 1 : -1);
         double f_lp, df_lp, d2f_lp;
-        fnc.eval<true, true>(lambda_pos, &f_lp, &df_lp, &d2f_lp);
+        fnc.secondAt(lambda_pos, &f_lp, &df_lp, &d2f_lp);
         f_pos = f_lp; df_pos = df_lp;
         nearShell |= d2f_lp < 0 &&
-            pow2(df_lp) - 2 * f_lp * d2f_lp - pow2(fnc.lambda * FUDGE_MINIMUM_RANGE * d2f_lp) < 0;
+            pow2(df_lp) - 2 * f_lp * d2f_lp - pow2(lambda * FUDGE_MINIMUM_RANGE * d2f_lp) < 0;
         if(nearShell || f_lp < 0)
-            lambda_min = lambda_max = fnc.lambda;
+            lambda_min = lambda_max = lambda;
     }
     if(!isFinite(lambda_min)) roots |= ROOT_LAMBDA_MIN;
     if(!isFinite(lambda_max)) roots |= ROOT_LAMBDA_MAX;
     rec.nuMax = nu_max; rec.lambdaMin = lambda_min; rec.lambdaMax = lambda_max;
     rec.nuUpper = nu_upper; rec.lambdaLower = lambda_lower; rec.lambdaPos = lambda_pos;
     rec.roots = roots;
-    if(ends) {
-        ends->fPos = f_pos; ends->dfPos = df_pos;
-        ends->fD2 = ends->dfD2 = ends->fNu = ends->dfNu = NAN;
-        if(((roots & ROOT_NU_MAX) && nu_upper == delta) || ((roots & ROOT_LAMBDA_MIN) && lambda_lower == delta))
-            fnc.eval<true, false>(delta, &ends->fD2, &ends->dfD2, nullptr);
-        if(roots & ROOT_NU_MAX)
-            fnc.eval<true, false>(fabs(fnc.nu), &ends->fNu, &ends->dfNu, nullptr);
-    }
+    ends->fPos = f_pos; ends->dfPos = df_pos;
+    ends->fD2 = ends->dfD2 = ends->fNu = ends->dfNu = NAN;
+    if(((roots & ROOT_NU_MAX) && nu_upper == delta) || ((roots & ROOT_LAMBDA_MIN) && lambda_lower == delta))
+        fnc.endD2(&ends->fD2, &ends->dfD2);
+    if(roots & ROOT_NU_MAX)
+        fnc.endNu(&ends->fNu, &ends->dfNu);
 }
 
 struct FudgeLimits { double lambda_min, lambda_max, nu_max; int order; };
@@ -313,49 +426,48 @@ static __device__ FudgeLimits fudgeLimitsFinish(const FudgeRecord& rec)
 
 /** One node of the momentum integral of sqrt(p^2(tau)) over [lo, hi] with the cubic end-point
     stretch (integrateGL of ScaledIntegrand<ScalingCub>(AxisymIntegrand), src/math_core.cpp:1191-1205,
-    src/actions_staeckel.cpp:276-299): the integrand times du/ds at the scaled node s. */
-static __device__ double fudgeMomentumNode(const FudgeFunction& fnc, double lo, double hi, double s)
+    src/actions_staeckel.cpp:276-299) at tau = lo + (hi - lo) s^2 (3 - 2 s): the integrand alone (the
+    node's weight and du/ds / (hi - lo) come tabulated). */
+__device__ __forceinline__ double fudgeMomentum(const MultipoleView& M, const FudgeBranch& f, double tau)
 {
-    double duds;
-    const double tau = unscaleCub(lo, hi, s, &duds);
-    const double tmd = tau - fnc.D2;
-    const double p2 = fnc.value(tau) / (2 * pow2(tmd) * tau);
-    double v = p2 < 0 ? 0 : sqrt(p2);
-    if(!isFinite(v)) v = 0;
-    return v * duds;
+    const double tmd = tau - f.D2;
+    const double p2 = f.value(M, tau) * rcpNormal(2 * pow2(tmd) * tau);
+    // p^2 < 0, NaN or infinite (a node on an end of the interval): no contribution
+    return p2 > 1e-280 && p2 < INFINITY ? p2 * rsqrtNormal(p2) : 0;
 }
 
 /** The same node with the integrand's arithmetic in FP32 (the mixed-precision form of the action
     quadrature): F(tau) and the point tau come from FP64 (the potential and the cancellation in
-    F stay FP64), then p = sqrt(F / (2 tau)) / |tau - D2| (the square root through the hardware
-    reciprocal square root) and the product with du/ds are FP32; the caller accumulates the weighted
-    terms with compensation. */
-static __device__ float fudgeMomentumNode32(const FudgeFunction& fnc, double lo, double hi, double s)
+    F stay FP64), then p = sqrt(F / (2 tau)) / |tau - D2| is FP32 (the square root through the hardware
+    reciprocal square root); the caller accumulates the weighted terms with compensation. */
+__device__ __forceinline__ float fudgeMomentum32(const MultipoleView& M, const FudgeBranch& f, double tau)
 {
-    double duds;
-    const double tau = unscaleCub(lo, hi, s, &duds);
-    const double F = fnc.value(tau);
+    const double F = f.value(M, tau), tmd64 = tau - f.D2;
     // p = sqrt(F / (2 tau)) / |tau - D2|: the square root before the division by (tau - D2)^2
     // keeps every FP32 intermediate in range for tau up to ~1e18 (the product (tau - D2)^2 tau
     // overflows FP32 already at tau ~ 1e12, where loosely bound orbits reach); a value of F
     // beyond the FP32 range takes the FP64 form
-    if(!(fabs(F) < 1e37)) return static_cast<float>(fudgeMomentumNode(fnc, lo, hi, s));
-    const float tmd = static_cast<float>(tau - fnc.D2), t = static_cast<float>(tau);
+    if(!(fabs(F) < 1e37)) {
+        const double p2 = F / (2 * pow2(tmd64) * tau), v = p2 < 0 ? 0 : sqrt(p2);
+        return isFinite(v) ? static_cast<float>(v) : 0.f;
+    }
+    const float tmd = static_cast<float>(tmd64), t = static_cast<float>(tau);
     const float q = static_cast<float>(F) / (2.f * t);
-    float v = q > 0.f ? q * rsqrtf(q) / fabsf(tmd) : 0.f;
-    if(!(v < INFINITY)) v = 0.f;
-    return v * static_cast<float>(duds);
+    const float v = q > 0.f ? q * rsqrtf(q) / fabsf(tmd) : 0.f;
+    return v < INFINITY ? v : 0.f;
 }
 
 /** Phase 1 of the actions of one point (R, z, phi, vR, vz, vphi) for focal distance fd
     (evalAxisymFudge, src/actions_staeckel.cpp:683-693: fd <= 0 falls back to max(R,1)*1e-4);
-    Phi is the potential at the point.  Writes Jphi into act[2]; for a point without actions
+    p has been located at the point.  Out of line, like locate(): one copy for
+    the kernels of given and of tabulated focal distances, so that both give the same bits.  Writes Jphi into act[2]; for a point without actions
     (unbound, or lambda = nu = Delta^2) also NaN into act[0..1] and marks the record invalid.
     Otherwise the record holds the integrals of motion (findIntegralsOfMotionAxisymFudge,
     :176-195) and the limits and root brackets of fudgeLimitsSetup (ends: as there). */
-static __device__ void fudgePrepare(const MultipoleView& M, const double* pc, double Phi, double fd,
-    FudgeRecord& rec, double* act, FudgeEnds* ends = nullptr)
+static __device__ __noinline__ void fudgePrepare(const MultipoleView& M, const double* pc, CellPoint& p, double fd,
+    FudgeRecord& rec, double* act, FudgeEnds* ends)
 {
+    const double Phi = p.Phi;
     const double R = pc[0], z = pc[1], phi = pc[2], vR = pc[3], vz = pc[4], vphi = pc[5];
     if(fd <= 0) fd = fmax(R, 1.) * 1e-4;
     const double D2 = fd * fd;
@@ -376,198 +488,20 @@ static __device__ void fudgePrepare(const MultipoleView& M, const double* pc, do
     double absnu = 2 * D2 / (sum + sqD) * z2;
     if(absnu * 2 > D2) absnu = D2 - dmn; else dmn = D2 - absnu;
     if(sqD == 0) { act[0] = act[1] = NAN; return; }   // lambda = nu = Delta^2: undefined
-    FudgeFunction fnc;
-    fnc.M = &M;
-    fnc.lambda = lambda;
-    fnc.nu = absnu * signz;
-    fnc.phi = 0;                    // axisymmetric potential: its evaluators never read the azimuth
-    fnc.D2 = D2;
-    fnc.bad = 0;
-    double Phi0;
-    CylDerivs g; CylHess h;
-    evalMultipoleCylCall<1, EVAL_AXI>(M, sqrt(lambda - D2), 0, 0, &Phi0, &g, &h);
+    const double Phi0 = p.equatorial(M, lambda - D2);
     const double Ekin = 0.5 * (vR * vR + vz * vz + vphi * vphi);
-    fnc.E = Phi + Ekin;
-    fnc.Lz = Lz;
-    fnc.flambda = -lambda * Phi0;
-    fnc.fnu = fnc.flambda + Phi * (lambda - absnu);
-    fnc.I3 = lambda * (Phi - Phi0) + 0.5 * (pow2(z * vphi) + pow2(R * vz - z * vR) + pow2(vz) * D2);
-    fnc.derive();
-    if(!isFinite(fnc.E + fnc.I3 + fnc.Lz) || fnc.E >= 0) { act[0] = act[1] = NAN; return; }
-    rec.lambda = fnc.lambda; rec.nu = fnc.nu; rec.D2 = D2; rec.E = fnc.E; rec.Lz = Lz; rec.I3 = fnc.I3;
-    rec.flambda = fnc.flambda; rec.fnu = fnc.fnu; rec.phi = phi;
-    fudgeLimitsSetup(fnc, rec, ends);
+    rec.lambda = lambda; rec.nu = absnu * signz; rec.D2 = D2; rec.E = Phi + Ekin; rec.Lz = Lz; rec.phi = phi;
+    rec.flambda = -lambda * Phi0;
+    rec.fnu = rec.flambda + Phi * (lambda - absnu);
+    rec.I3 = lambda * (Phi - Phi0) + 0.5 * (pow2(z * vphi) + pow2(R * vz - z * vR) + pow2(vz) * D2);
+    if(!isFinite(rec.E + rec.I3 + rec.Lz) || rec.E >= 0) { act[0] = act[1] = NAN; return; }
+    p.rec = &rec;
+    fudgeLimitsSetup(p, rec, ends);
     // velocities in prolate spheroidal coordinates (src/coord.cpp:317-322, :525-531)
     const double lambdadot = R * 2 * lambda / sqD * vR + z * 2 * lmd / sqD * vz;
     const double nudot = R * 2 * -absnu / sqD * signz * vR + z * 2 * dmn / sqD * signz * vz;
-    rec.valid = REC_VALID | (lambdadot >= 0 ? REC_LDOT_POS : 0) | (nudot * fnc.nu >= 0 ? REC_NDOT_NU_POS : 0) |
+    rec.valid = REC_VALID | (lambdadot >= 0 ? REC_LDOT_POS : 0) | (nudot * rec.nu >= 0 ? REC_NDOT_NU_POS : 0) |
         (nudot < 0 ? REC_NUDOT_NEG : 0);
-}
-
-/** Inverse of the cubic end-point scaling (math::scale of ScalingCub, src/math_core.cpp:370-386):
-    s in [0, 1] with u = ul (1-s)^2 (1+2s) + ur s^2 (3-2s).  On the nearer half, w = s^2 (3 - 2s) is
-    a depressed cubic in y = s - 1/2 whose trigonometric root s = 1/2 + cos((acos(1 - 2w) - 2pi)/3)
-    is polished by three Newton steps; u outside [ul, ur] gives NaN, as in the reference. */
-static __device__ double scaleCubInverse(double ul, double ur, double u)
-{
-    if(u == ul) return 0;
-    if(u == ur) return 1;
-    const double half = 0.5 * (ul + ur);
-    if(u == half) return 0.5;
-    const double w = u < half ? (u - ul) / (ur - ul) : (ur - u) / (ur - ul);
-    double s = 0.5 + cos((acos(1 - 2 * w) - 2 * M_PI) / 3);
-    for(int i = 0; i < 3; i++)
-        s -= (s * s * (3 - 2 * s) - w) / (6 * s * (1 - s));
-    return u < half ? s : 1 - s;
-}
-
-/// the three integrands of AxisymIntegrand::value with p in the denominator (n = -1), from one
-/// F(tau): (tau-Delta^2)^-1 [E], (tau-Delta^2)^-1 tau^-1 [I3], (tau-Delta^2)^-2 with the singular
-/// part at nu_max removed [Lz] (src/actions_staeckel.cpp:276-299)
-struct InverseMomentumTerms { double e, i3, lz; };
-
-static __device__ InverseMomentumTerms inverseMomentumTerms(double ft, double tau, double D2, double nuMax,
-    double dfdnuMax)
-{
-    InverseMomentumTerms t{ 0, 0, 0 };
-    const double tmd = tau - D2;
-    const double p2 = ft / (2 * pow2(tmd) * tau);
-    if(p2 < 0) return t;
-    const double r = 1 / sqrt(p2);
-    double v = r / tmd;
-    t.e = isFinite(v) ? v : 0;
-    v = r / tmd / tau;
-    t.i3 = isFinite(v) ? v : 0;
-    v = r / pow2(tmd);
-    if(tmd < 0) v += sqrt(2 * nuMax / dfdnuMax / (tau - nuMax)) / tmd;
-    t.lz = isFinite(v) ? v : 0;
-    return t;
-}
-
-/// GL rule of the requested order (the next tabulated one at or above it)
-static __device__ __forceinline__ int glRule(const GLRules& gl, int order, const double** x, const double** w)
-{
-    int N = order < 1 ? 1 : order;
-    while(gl.offset[N] < 0) N++;
-    *x = gl.nodes + gl.offset[N];
-    *w = gl.weights + gl.offset[N];
-    return N;
-}
-
-/** the inverse-momentum integrals of one branch over the scaled interval [0, y] of [lo, hi]
-    (integrateGL(ScaledIntegrand<ScalingCub>, 0, y, N), src/math_core.cpp:1191-1205); with
-    ACT also the action integral (p in the numerator) over the same nodes, when y = 1 */
-template<bool ACT>
-static __device__ InverseMomentumTerms branchIntegrals(const FudgeFunction& fnc, const GLRules& gl, int order,
-    double lo, double hi, double y, double nuMax, double dfdnuMax, double* act)
-{
-    InverseMomentumTerms sum{ 0, 0, 0 };
-    if(ACT) *act = 0;
-    if(y == 0) return sum;
-    const double *x, *w;
-    const int N = glRule(gl, order, &x, &w);
-    double sa = 0;
-    for(int i = 0; i < N; i++) {
-        const double xi = ldg(x + i), wi = ldg(w + i);
-        double duds;
-        const double tau = unscaleCub(lo, hi, y * xi + 0 * (1 - xi), &duds);
-        const double ft = fnc.value(tau);
-        const InverseMomentumTerms t = inverseMomentumTerms(ft, tau, fnc.D2, nuMax, dfdnuMax);
-        sum.e += wi * (t.e * duds);
-        sum.i3 += wi * (t.i3 * duds);
-        sum.lz += wi * (t.lz * duds);
-        if(ACT) {
-            const double tmd = tau - fnc.D2;
-            const double p2 = ft / (2 * pow2(tmd) * tau);
-            double v = p2 < 0 ? 0 : sqrt(p2);
-            if(!isFinite(v)) v = 0;
-            sa += wi * (v * duds);
-        }
-    }
-    sum.e *= y; sum.i3 *= y; sum.lz *= y;
-    if(ACT) *act = sa * y;
-    return sum;
-}
-
-/// 2 pi wrap of an angle into [0, 2 pi) (math::wrapAngle, src/math_core.cpp:149-157; NaN -> 0)
-static __device__ __forceinline__ double wrapAngle(double x)
-{
-    x -= 2 * M_PI * floor(1 / (2 * M_PI) * x);
-    return x >= 0 && x < 2 * M_PI ? x : 0;
-}
-
-/** Actions, frequencies and angles of a prepared point whose roots are found (evalAxisym,
-    src/actions_staeckel.cpp:645-670): computeActions (:604-619), computeActionDerivatives
-    (:489-527), computeIntDerivatives (:532-560), computeGenFuncDerivatives (:566-600) and
-    computeAngles (:624-636).  The action integrals and the derivative integrals share their
-    potential evaluations (same nodes); ang / freq may be null. */
-static __device__ void fudgeAnglesFrequencies(const MultipoleView& M, const GLRules& gl, const FudgeRecord& rec,
-    double* act, double* ang, double* freq)
-{
-    FudgeFunction fnc;
-    loadFudgeFunction(M, rec, fnc);
-    const FudgeLimits lim = fudgeLimitsFinish(rec);
-    const double D2 = rec.D2, Lz = rec.Lz;
-    double dfdnuMax, unused;
-    fnc.eval<true, false>(lim.nu_max, &unused, &dfdnuMax, nullptr);
-    // action derivatives over (E, I3, Lz), full ranges; the actions from the same nodes
-    double Jr, Jz;
-    InverseMomentumTerms L = branchIntegrals<true>(fnc, gl, lim.order, lim.lambda_min, lim.lambda_max, 1,
-        lim.nu_max, dfdnuMax, &Jr);
-    const InverseMomentumTerms N = branchIntegrals<true>(fnc, gl, lim.order, 0, lim.nu_max, 1,
-        lim.nu_max, dfdnuMax, &Jz);
-    act[0] = Jr / M_PI;
-    act[1] = Jz / M_PI * 2;
-    if(lim.lambda_min == lim.lambda_max) {      // limitingIntegralValue, :307-323
-        const double tau = lim.lambda_min, tmd = tau - D2;
-        double d2, v0;
-        fnc.eval<false, true>(tau, &v0, nullptr, &d2);
-        const double base = 2 * M_PI * sqrt(-tau / d2) * fabs(tmd);
-        L.e = base / tmd;
-        L.i3 = base / tmd / tau;
-        L.lz = base / pow2(tmd);
-    }
-    const double dJrdE = L.e / (4 * M_PI), dJzdE = N.e / (2 * M_PI);
-    const double dJrdI3 = -L.i3 / (4 * M_PI), dJzdI3 = -N.i3 / (2 * M_PI);
-    const double dJrdLz = -Lz * L.lz / (4 * M_PI);
-    const double dmn = D2 - lim.nu_max;
-    const double singpart = 2 * sqrt(-2 * lim.nu_max / dfdnuMax / dmn) * atan(sqrt(lim.nu_max / dmn));
-    const double dJzdLz = -Lz * (N.lz + singpart) / (2 * M_PI);
-    // inverse matrix: frequencies and the derivatives of I3 over the actions
-    double Or, Oz, Ophi, dI3dJr, dI3dJz, dI3dJphi;
-    const double det = dJrdE * dJzdI3 - dJrdI3 * dJzdE;
-    if(lim.nu_max == 0 || det == 0) {
-        Or = 1 / dJrdE;
-        Ophi = -dJrdLz / dJrdE;
-        dI3dJr = dI3dJz = dI3dJphi = Oz = 0;
-    } else {
-        Or = dJzdI3 / det;
-        Oz = -dJrdI3 / det;
-        Ophi = (dJrdI3 * dJzdLz - dJrdLz * dJzdI3) / det;
-        dI3dJr = -dJzdE / det;
-        dI3dJz = dJrdE / det;
-        dI3dJphi = -(dJrdE * dJzdLz - dJrdLz * dJzdE) / det;
-    }
-    if(freq) { freq[0] = Or; freq[1] = Oz; freq[2] = Ophi; }
-    if(!ang) return;
-    // derivatives of the generating function over (E, I3, Lz): integrals up to the point
-    const double signl = rec.valid & REC_LDOT_POS ? 1 : -1, signn = rec.valid & REC_NDOT_NU_POS ? 1 : -1;
-    const double absnu = fabs(rec.nu);
-    const double yl = scaleCubInverse(lim.lambda_min, lim.lambda_max, rec.lambda);
-    const double yn = lim.nu_max == 0 ? 0 : scaleCubInverse(0, lim.nu_max, absnu);
-    const InverseMomentumTerms Lp = branchIntegrals<false>(fnc, gl, lim.order, lim.lambda_min, lim.lambda_max, yl,
-        lim.nu_max, dfdnuMax, nullptr);
-    const InverseMomentumTerms Np = branchIntegrals<false>(fnc, gl, lim.order, 0, lim.nu_max, yn,
-        lim.nu_max, dfdnuMax, nullptr);
-    const double dSdE = signl * Lp.e / 4 + signn * Np.e / 4;
-    const double dSdI3 = signl * -Lp.i3 / 4 + signn * -Np.i3 / 4;
-    const double singS = 2 * sqrt(-2 * lim.nu_max / dfdnuMax / dmn) *
-        (atan(sqrt(lim.nu_max / dmn)) - atan(sqrt((lim.nu_max - absnu) / dmn)));
-    const double dSdLz = Lz == 0 ? 0 : rec.phi + signl * -Lz * Lp.lz / 4 + signn * -Lz * (Np.lz + singS) / 4;
-    const bool addPi = (rec.valid & REC_NUDOT_NEG) && Lz != 0;
-    ang[0] = wrapAngle(dSdE * Or + dSdI3 * dI3dJr + dSdLz * 0);
-    ang[1] = wrapAngle(dSdE * Oz + dSdI3 * dI3dJz + dSdLz * 0 + M_PI * addPi);
-    ang[2] = wrapAngle(dSdE * Ophi + dSdI3 * dI3dJphi + dSdLz * 1);
 }
 
 /// Cartesian posvel -> cylindrical (R, z, phi, vR, vz, vphi); reference src/coord.cpp:476-484
@@ -589,7 +523,7 @@ __device__ __forceinline__ void carToCylPosVel(const double* w, double* pc)
 /** focal distance of the action finder at a point with potential Phi: E, Lz -> Lcirc(E) ->
     (xi, chi) -> Delta; reference ActionFinderAxisymFudge::eval steps 0-1,
     src/actions_staeckel.cpp:957-977 */
-static __device__ double finderFocalDistance(const FudgeTables& F, const double* pc, double Phi)
+static __device__ __forceinline__ double finderFocalDistance(const FudgeTables& F, const double* pc, double Phi)
 {
     const double E = Phi + 0.5 * (pc[3] * pc[3] + pc[4] * pc[4] + pc[5] * pc[5]);
     const double Lz = pc[0] * pc[5];
@@ -598,6 +532,19 @@ static __device__ double finderFocalDistance(const FudgeTables& F, const double*
     const double Lzrel = clip(fabs(Lz) / Lcirc, 0., 1.);
     const double chi = scaleCub(0, 1, Lzrel);
     return fmax(0., deltaLookup(F, xi, chi));
+}
+
+/// inputs of the bracket predictor: the point's (R, z, vR, vz, vphi) with E and Lz in
+/// scale-free form -- ln r, |z| / r, velocities over the escape speed sqrt(-2 Phi) (so
+/// that E = Phi (1 - v^2 / v_esc^2) and Lz = R vphi follow), ln(Delta / r); symmetric
+/// under z -> -z and Lz -> -Lz like the limits themselves
+__device__ __forceinline__ void bracketFeatures(const double* pc, double Phi, double delta, float* out)
+{
+    const double r = fmax(sqrt(pc[0] * pc[0] + pc[1] * pc[1]), 1e-300), vesc = sqrt(fmax(-2 * Phi, 1e-300));
+    const float f[6] = { static_cast<float>(log(r)), static_cast<float>(fabs(pc[1]) / r),
+        static_cast<float>(pc[3] / vesc), static_cast<float>((pc[1] >= 0 ? pc[4] : -pc[4]) / vesc),
+        static_cast<float>(fabs(pc[5]) / vesc), static_cast<float>(log(fmax(delta, 1e-300) / r)) };
+    for(int k = 0; k < 6; k++) out[k] = f[k];
 }
 
 }  // namespace agb

@@ -1,7 +1,7 @@
 // Phase 3 of the Staeckel-fudge computation when angles or frequencies are requested: actions,
 // frequencies and angles of each prepared point, one point per thread.
 #include "runtime.h"
-#include "fudge.cuh"
+#include "fudge_nodes.cuh"
 #include "fudge_phases.h"
 
 namespace agb {

@@ -14,15 +14,22 @@ struct FudgeEnds;
 /// kinds: nu_max, lambda_min, lambda_max)
 struct BracketWidths { float w[3]; };
 
+/// phase 1 from the node form of the splines, for calls with angles, frequencies or focal distances
+/// (the focal distance handed to the caller is that of the calls with angles, so that passing it
+/// back gives the same angles); arguments as those of fudgePrepareKernel
+void launchNodePrepare(bool finder, const MultipoleView& M, const FudgeTables& F, long n, const double* posvel,
+    const double* fd, double fd0, FudgeRecord* rec, double* act, double* fdOut, int* iters, float* features,
+    FudgeEnds* ends, cudaStream_t stream);
+
 /// phase 2: the root searches of the integration limits, drained by a persistent grid from a
 /// device work counter (8 bytes, zeroed here on the stream); with pred (n x 3 predictions) the
 /// searches start on the predicted brackets; stats (4 counters, may be null) accumulates
 /// searches, narrowed searches, fallbacks to the plain bracket and iterations; ends (may be null):
 /// F and F' at the ends of each record's plain brackets, which the plain searches take instead of
-/// evaluating them again
+/// evaluating them again; nodes: F from the node form of the splines (records whose angles follow)
 void launchFudgeRoots(const MultipoleView& M, long n, FudgeRecord* rec, const FudgeEnds* ends, int* iters,
     unsigned long long* counter, const float* pred, const BracketWidths& widths, unsigned long long* stats,
-    cudaStream_t stream);
+    bool nodes, cudaStream_t stream);
 
 /// training targets of the bracket predictor from records whose plain searches are done
 void launchBracketTargets(long n, const FudgeRecord* rec, float* target, float* mask, cudaStream_t stream);

@@ -2,11 +2,12 @@
 // own compilation unit so that its register budget does not constrain the other phases (the
 // potential evaluator is a non-inlined function compiled once per unit).
 #include "runtime.h"
-#include "fudge.cuh"
+#include "fudge_nodes.cuh"
 #include "fudge_phases.h"
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <type_traits>
 
 namespace agb {
 
@@ -16,9 +17,9 @@ constexpr int ROOT_BLOCK = 128;
 constexpr unsigned FULL_MASK = 0xffffffffu;
 
 /// the limit found by a plain search (nu_max falls back to |nu| when the search found no root)
-__device__ __forceinline__ void storePlainLimit(FudgeRecord& r, int kind, const RootSearch& s, double u0, double nu)
+__device__ __forceinline__ void storePlainLimit(FudgeRecord& r, int kind, const RootSearch& s, double u0)
 {
-    if(kind == ROOT_NU_MAX) r.nuMax = isFinite(s.result) ? s.result : fabs(nu);
+    if(kind == ROOT_NU_MAX) r.nuMax = isFinite(s.result) ? s.result : fabs(r.nu);
     else if(kind == ROOT_LAMBDA_MIN) r.lambdaMin = s.result;
     else r.lambdaMax = unscaleSemiInf(u0, s.result, nullptr);
 }
@@ -102,8 +103,9 @@ __device__ __forceinline__ bool predictedBracket(const FudgeRecord& r, int kind,
     be null) accumulates {searches, seeded searches, plain searches after a failed check,
     iterations} when STATS.  LEARNED = false (no predictions, no stats) compiles the plain searches
     alone, without that state and the counters (fewer registers); STATS = false leaves the
-    counters out of the learned searches. */
-template<bool LEARNED, bool STATS>
+    counters out of the learned searches.  NODES = true evaluates F from the node form of the splines
+    (points whose angles follow), false from the cells. */
+template<bool LEARNED, bool STATS, bool NODES>
 __global__ void __launch_bounds__(ROOT_BLOCK, 4) fudgeRootKernel(const __grid_constant__ MultipoleView M, long n,
     FudgeRecord* __restrict__ rec, const FudgeEnds* __restrict__ ends, int* __restrict__ iters,
     unsigned long long* __restrict__ counter, const float* __restrict__ pred, const BracketWidths widths,
@@ -117,7 +119,7 @@ __global__ void __launch_bounds__(ROOT_BLOCK, 4) fudgeRootKernel(const __grid_co
     int kind = 0;
     double x = 0, u0 = 0, verified = 0;
     unsigned nSearch = 0, nSeeded = 0, nFallback = 0, nIter = 0;
-    FudgeFunction fnc;
+    std::conditional_t<NODES, FudgeFunction, FudgeBranch> fnc{};
     RootSearch s;
     // a plain search on the point's bracket again (after a seeded root failed its check)
     auto restartPlain = [&]() {
@@ -129,7 +131,7 @@ __global__ void __launch_bounds__(ROOT_BLOCK, 4) fudgeRootKernel(const __grid_co
         if(STATS) nFallback++;
         mode = setupPlain(s, kind, ends ? ends + point : nullptr, lo, hi, fabs(lo - hi) * FUDGE_ACCURACY_RANGE,
                           u0, fnc.D2, fnc.E, &x);
-        if(mode == LANE_IDLE) storePlainLimit(rec[point], kind, s, u0, fnc.nu);
+        if(mode == LANE_IDLE) storePlainLimit(rec[point], kind, s, u0);
     };
     // the search has ended with s.result: store the limit, or (a seeded search) check its root
     auto finishSearch = [&]() {
@@ -152,7 +154,7 @@ __global__ void __launch_bounds__(ROOT_BLOCK, 4) fudgeRootKernel(const __grid_co
             return;
         }
         mode = LANE_IDLE;
-        storePlainLimit(rec[point], kind, s, u0, fnc.nu);
+        storePlainLimit(rec[point], kind, s, u0);
         if(iters) atomicAdd(iters + point, s.iter);
     };
     while(true) {
@@ -175,7 +177,8 @@ __global__ void __launch_bounds__(ROOT_BLOCK, 4) fudgeRootKernel(const __grid_co
                     if(r.roots & (1 << k)) {
                         point = i;
                         kind = 1 << k;
-                        loadFudgeFunction(M, r, fnc);
+                        if constexpr(NODES) loadFudgeFunction(M, r, fnc);
+                        else loadFudgeBranch(r, kind != ROOT_NU_MAX, fnc);
                         u0 = r.lambdaPos;
                         const double lo = kind == ROOT_NU_MAX ? fabs(r.nu) : kind == ROOT_LAMBDA_MIN ? r.lambdaLower : 0;
                         const double hi = kind == ROOT_NU_MAX ? r.nuUpper : kind == ROOT_LAMBDA_MIN ? r.lambdaPos : 1;
@@ -184,7 +187,7 @@ __global__ void __launch_bounds__(ROOT_BLOCK, 4) fudgeRootKernel(const __grid_co
                         mode = setupPlain(s, kind, ends ? ends + i : nullptr, lo, hi, tol, u0, r.D2, r.E, &x);
                         fresh = mode == LANE_PROPOSE;
                         if(mode == LANE_IDLE)       // no sign change or a root at an end
-                            storePlainLimit(rec[i], kind, s, u0, fnc.nu);
+                            storePlainLimit(rec[i], kind, s, u0);
                         if(STATS) nSearch++;
                     }
                 }
@@ -228,7 +231,10 @@ __global__ void __launch_bounds__(ROOT_BLOCK, 4) fudgeRootKernel(const __grid_co
         }
         // 3. F (and F') at the points of the lanes that have one
         double fx = 0, dx = 0;
-        if(mode == LANE_EVAL || mode == LANE_VERIFY) limitRootEval(fnc, kind, u0, x, &fx, &dx);
+        if(mode == LANE_EVAL || mode == LANE_VERIFY) {
+            if constexpr(NODES) limitRootEval(fnc, kind, u0, x, &fx, &dx);
+            else limitRootEval(M, fnc, kind == ROOT_LAMBDA_MAX, u0, x, &fx, &dx);
+        }
         // 4. the values fed to the searches
         if(mode == LANE_EVAL) {
             const int r = s.take(fx, dx, &x);
@@ -283,7 +289,7 @@ __global__ void bracketTargetKernel(long n, const FudgeRecord* __restrict__ rec,
 }
 
 /// resident blocks of a root-kernel variant on the current device (cached per device and variant)
-template<bool LEARNED, bool STATS>
+template<bool LEARNED, bool STATS, bool NODES>
 int rootGridSize()
 {
     static std::mutex mutex;
@@ -295,7 +301,7 @@ int rootGridSize()
     if(it != cache.end()) return it->second;
     int sms = 0, perSM = 0;
     AGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    AGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, fudgeRootKernel<LEARNED, STATS>, ROOT_BLOCK, 0));
+    AGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, fudgeRootKernel<LEARNED, STATS, NODES>, ROOT_BLOCK, 0));
     const int grid = std::max(1, sms * std::max(1, perSM));
     cache[dev] = grid;
     return grid;
@@ -303,26 +309,31 @@ int rootGridSize()
 
 }  // namespace
 
-void launchFudgeRoots(const MultipoleView& M, long n, FudgeRecord* rec, const FudgeEnds* ends, int* iters,
+namespace {
+template<bool LEARNED, bool STATS, bool NODES>
+void launchRoots(const MultipoleView& M, long n, FudgeRecord* rec, const FudgeEnds* ends, int* iters,
     unsigned long long* counter, const float* pred, const BracketWidths& widths, unsigned long long* stats,
     cudaStream_t stream)
 {
+    const long tasks = (3 * n + ROOT_BLOCK - 1) / ROOT_BLOCK;
+    const long grid = std::min<long>(rootGridSize<LEARNED, STATS, NODES>(), tasks);
+    fudgeRootKernel<LEARNED, STATS, NODES><<<grid, ROOT_BLOCK, 0, stream>>>(M, n, rec, ends, iters, counter, pred, widths,
+        stats);
+    AGB_CUDA(cudaGetLastError());
+}
+}  // namespace
+
+void launchFudgeRoots(const MultipoleView& M, long n, FudgeRecord* rec, const FudgeEnds* ends, int* iters,
+    unsigned long long* counter, const float* pred, const BracketWidths& widths, unsigned long long* stats,
+    bool nodes, cudaStream_t stream)
+{
     if(n <= 0) return;
     AGB_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), stream));
-    const long tasks = (3 * n + ROOT_BLOCK - 1) / ROOT_BLOCK;
-    if(stats) {              // learned or plain searches with the counters
-        const long grid = std::min<long>(rootGridSize<true, true>(), tasks);
-        fudgeRootKernel<true, true><<<grid, ROOT_BLOCK, 0, stream>>>(M, n, rec, ends, iters, counter, pred, widths, stats);
-    } else if(pred) {
-        const long grid = std::min<long>(rootGridSize<true, false>(), tasks);
-        fudgeRootKernel<true, false><<<grid, ROOT_BLOCK, 0, stream>>>(M, n, rec, ends, iters, counter, pred, widths,
-            nullptr);
-    } else {
-        const long grid = std::min<long>(rootGridSize<false, false>(), tasks);
-        fudgeRootKernel<false, false><<<grid, ROOT_BLOCK, 0, stream>>>(M, n, rec, ends, iters, counter, nullptr, widths,
-            nullptr);
-    }
-    AGB_CUDA(cudaGetLastError());
+    // learned or plain searches with the counters; predictions alone; plain searches
+    auto launch = stats ? (nodes ? launchRoots<true, true, true> : launchRoots<true, true, false>)
+                : pred  ? (nodes ? launchRoots<true, false, true> : launchRoots<true, false, false>)
+                        : (nodes ? launchRoots<false, false, true> : launchRoots<false, false, false>);
+    launch(M, n, rec, ends, iters, counter, pred, widths, stats, stream);
 }
 
 void launchBracketTargets(long n, const FudgeRecord* rec, float* target, float* mask, cudaStream_t stream)

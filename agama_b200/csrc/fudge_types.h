@@ -7,11 +7,14 @@ namespace agb {
 constexpr int GL_MAX_ORDER = 40;                 // reference MAX_GL_ORDER, src/math_core.h:577
 
 /// Gauss-Legendre rules on [0, 1] for the orders the reference tabulates (1..20, 25, 32, 40):
-/// nodes and weights of rule n start at offset[n]; orders without a rule map to the next one
+/// nodes and weights of rule n start at offset[n]; orders without a rule map to the next one.
+/// cubic: pairs (s^2 (3 - 2 s), w 6 s (1 - s)), i.e. the nodes under the cubic end-point stretch of a
+/// unit interval and their weights times its derivative
 struct GLRules {
     int offset[GL_MAX_ORDER + 1];   // -1 where no rule
     const double* nodes;
     const double* weights;
+    const double* cubic;
 };
 
 /// 1-D quintic spline stored as [x | f | f' | f''] with n nodes each

@@ -50,7 +50,7 @@ __device__ __forceinline__ void ldg4(const double* p, double* v)
 /// index, nodes and reciprocal width.  For x outside or NaN the result is some cell of the grid.
 __device__ __forceinline__ int gridCell(const GridView& g, double x, double* xl, double* xh, double* invH)
 {
-    const int b = min(max(static_cast<int>((x - g.x0) * g.lutScale), 0), g.nlut - 1);
+    const int b = min(max(__double2int_rz((x - g.x0) * g.lutScale), 0), g.nlut - 1);
     int k = __ldg(g.lut + b);
     double2 lo = ldg2(&g.cell[k].x), hi = ldg2(&g.cell[k + 1].x);
     while(x >= hi.x && k < g.n - 2) {
