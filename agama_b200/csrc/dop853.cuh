@@ -1,7 +1,7 @@
 // DOP853 orbit integration on the device: one orbit per thread, Runge-Kutta stage vectors in
 // shared memory (thread-interleaved, bank-conflict free), state and step control in registers.
 #pragma once
-#include "multipole_eval.cuh"
+#include "multipole_force.cuh"
 
 namespace agb {
 
@@ -153,22 +153,22 @@ constexpr double fdec = 0.333, finc = 6.0, safe = 0.9;   // step-size control
     min(1, |E| / max(|Phi|, K)).  Reference OrbitIntegrator<Car>::eval, src/orbit.cpp:183-208.
     G > 1: called together by a group of G lanes with the same point, which share the spline
     evaluations (the multi-harmonic evaluator kind only). */
-template<int NQ, int KIND, int G = 1, bool MIXED = false>
+template<int KIND, int G = 1, bool MIXED = false>
 __device__ __forceinline__ void orbitRHS(const MultipoleView& M, double Omega, double time,
     const double* xv, double* dxdt, double* accFac)
 {
     double ca = 1, sa = 0;
     if(Omega != 0) sincos(Omega * time, &sa, &ca);
-    double Epot, g[3], h[6];
-    evalMultipoleCar<NQ, KIND, G, MIXED>(M, xv[0] * ca + xv[1] * sa, xv[1] * ca - xv[0] * sa, xv[2], &Epot, g, h);
+    double Epot, g[3];
+    evalForceCar<KIND, G, MIXED>(M, sumProducts(xv[0], ca, xv[1], sa), sumProducts(xv[1], ca, -xv[0], sa), xv[2], &Epot, g);
     dxdt[0] = xv[3];
     dxdt[1] = xv[4];
     dxdt[2] = xv[5];
-    dxdt[3] = -g[0] * ca + g[1] * sa;
-    dxdt[4] = -g[1] * ca - g[0] * sa;
+    dxdt[3] = sumProducts(g[1], sa, -g[0], ca);
+    dxdt[4] = sumProducts(-g[1], ca, -g[0], sa);
     dxdt[5] = -g[2];
     if(accFac) {
-        const double Ekin = 0.5 * (xv[3] * xv[3] + xv[4] * xv[4] + xv[5] * xv[5]);
+        const double Ekin = 0.5 * fma(xv[5], xv[5], sumProducts(xv[3], xv[3], xv[4], xv[4]));
         *accFac = fmin(1., fabs(Epot + Ekin) / fmax(fabs(Epot), Ekin));
     }
 }

@@ -40,6 +40,7 @@ struct PowerLawView {
     const double* S;      // slopes, (lmax+1)^2
     const double* U;      // amplitudes of (r/r0)^s
     const double* W;      // amplitudes of (r/r0)^v
+    const double* norm;   // [m][l]: sqrt((2l+1)/(2l-1) (l-m)/(l+m)), stride LMAX_MAX + 1
 };
 
 /** device view of one grid of the 2-D splines, for the search of the cell that holds a value: cell

@@ -35,14 +35,17 @@ struct StageStore {
 
 /// The Runge-Kutta stages of one DOP853 attempt as table rows: row r forms the point of stage
 /// r+2 (k_{r+2}) as x + h sum coef * k_src, row 11 the 8th-order solution (weights b).  Sources:
-/// -1 = k1 (registers), otherwise a stage slot; results go to slot dest[r].  Terms and their order
-/// are those of OdeStepperDOP853::doStep (src/math_ode.cpp:243-300); unused terms have coef 0.
+/// -1 = k1 (registers), otherwise a stage slot; the result of row r goes to slot r (r - 9 for k11 and
+/// k12, which take the places of k2 and k3).  Terms and their order are those of
+/// OdeStepperDOP853::doStep (src/math_ode.cpp:243-300).
 constexpr int NUM_ROWS = 12, MAX_TERMS = 9, K1 = -1;
+constexpr int INIT_ROW = NUM_ROWS - 3;               // row at which a new orbit's three evaluations begin
+constexpr unsigned FULL_MASK = 0xffffffffu;
 struct StageTable {
     double coef[NUM_ROWS][MAX_TERMS];
     double c[NUM_ROWS];
     signed char src[NUM_ROWS][MAX_TERMS];
-    signed char dest[NUM_ROWS];
+    int terms[NUM_ROWS];
 };
 
 __host__ __device__ constexpr StageTable makeStageTable()
@@ -68,14 +71,13 @@ __host__ __device__ constexpr StageTable makeStageTable()
         { K1, 2, 3, 4, 5, 6, 7, 8, 0 }, { K1, 4, 5, 6, 7, 8, 0, 1 } };
     const int nterms[NUM_ROWS] = { 1, 2, 2, 3, 3, 4, 5, 6, 7, 8, 9, 8 };
     const double c[NUM_ROWS] = { c2, c3, c4, c5, c6, c7, c8, c9, c10, c11, 1, 1 };
-    const signed char dest[NUM_ROWS] = { 0, 1, 2, 3, 4, 5, 6, 7, 8, 0, 1, -1 };
     for(int r = 0; r < NUM_ROWS; r++) {
         for(int t = 0; t < MAX_TERMS; t++) {
             T.coef[r][t] = t < nterms[r] ? coef[r][t] : 0;
             T.src[r][t] = t < nterms[r] ? src[r][t] : K1;
         }
         T.c[r] = c[r];
-        T.dest[r] = dest[r];
+        T.terms[r] = nterms[r];
     }
     return T;
 }
@@ -102,13 +104,13 @@ __device__ void denseOutput(double h, double offset, const double* x, const doub
             k11 = S.at(0, c), k12 = S.at(1, c);
         const double xd = xt[c] - x[c], xc = h * k1[c] - xd;
         const double r4 = xd - h * k13[c] - xc;
-        const double r5 = h * (d41 * k1[c] + d46 * k6 + d47 * k7 + d48 * k8 + d49 * k9 + d410 * k10 +
+        const double r5 = h * (sumProducts(d46, k6, d41, k1[c]) + d47 * k7 + d48 * k8 + d49 * k9 + d410 * k10 +
                                d411 * k11 + d412 * k12 + d413 * k13[c]);
-        const double r6 = h * (d51 * k1[c] + d56 * k6 + d57 * k7 + d58 * k8 + d59 * k9 + d510 * k10 +
+        const double r6 = h * (sumProducts(d51, k1[c], d56, k6) + d57 * k7 + d58 * k8 + d59 * k9 + d510 * k10 +
                                d511 * k11 + d512 * k12 + d513 * k13[c]);
-        const double r7 = h * (d61 * k1[c] + d66 * k6 + d67 * k7 + d68 * k8 + d69 * k9 + d610 * k10 +
+        const double r7 = h * (sumProducts(d61, k1[c], d66, k6) + d67 * k7 + d68 * k8 + d69 * k9 + d610 * k10 +
                                d611 * k11 + d612 * k12 + d613 * k13[c]);
-        const double r8 = h * (d71 * k1[c] + d76 * k6 + d77 * k7 + d78 * k8 + d79 * k9 + d710 * k10 +
+        const double r8 = h * (sumProducts(d76, k6, d71, k1[c]) + d77 * k7 + d78 * k8 + d79 * k9 + d710 * k10 +
                                d711 * k11);
         v[c] = x[c] + p * (xd + q * (xc + p * (r4 + q * (r5 + p * (r6 + q * (r7 + p * r8))))));
     }
@@ -120,11 +122,11 @@ __device__ __forceinline__ void toPotentialFrame(double Omega, double tabs, cons
 {
     double ca = 1, sa = 0;
     if(Omega != 0) sincos(Omega * tabs, &sa, &ca);
-    o[0] = v[0] * ca + v[1] * sa;
-    o[1] = v[1] * ca - v[0] * sa;
+    o[0] = sumProducts(v[0], ca, v[1], sa);
+    o[1] = sumProducts(v[1], ca, -v[0], sa);
     o[2] = v[2];
-    o[3] = v[3] * ca + v[4] * sa;
-    o[4] = v[4] * ca - v[3] * sa;
+    o[3] = sumProducts(v[3], ca, v[4], sa);
+    o[4] = sumProducts(v[4], ca, -v[3], sa);
     o[5] = v[5];
 }
 
@@ -167,14 +169,45 @@ __device__ void targetStep(const OrbitParams& P, long i, double t, double h, con
     }
 }
 
-/// phases of the per-lane integration state machine
-enum { PH_FETCH, PH_INIT1, PH_INIT2, PH_INIT3, PH_STAGE, PH_FINISH };
+/// the point of row `row` of an attempt: xt = x + h sum coef k over the row's terms, in their order
+/// (acc: the sum).  Rows of fewer than MAX_TERMS terms end with 0 k1, which leaves the sum as it is
+/// but for the sign of a zero and k1 that are not finite.
+template<int ROW>
+__device__ __forceinline__ void stagePoint(const StageStore& S, const double* x, const double* k1, double h, double* acc,
+    double* xt)
+{
+    constexpr StageTable T = makeStageTable();
+#pragma unroll
+    for(int c = 0; c < 6; c++) {
+        if(T.terms[ROW] == 1)
+            acc[c] = STAGE_TABLE.coef[ROW][0] * k1[c];
+        else
+            acc[c] = sumProducts(STAGE_TABLE.coef[ROW][0], k1[c], STAGE_TABLE.coef[ROW][1], S.at(T.src[ROW][1], c));
+#pragma unroll
+        for(int m = 2; m < T.terms[ROW]; m++) acc[c] = fma(STAGE_TABLE.coef[ROW][m], S.at(T.src[ROW][m], c), acc[c]);
+        if(T.terms[ROW] < MAX_TERMS) acc[c] = fma(0.0, k1[c], acc[c]);
+        xt[c] = fma(h, acc[c], x[c]);
+    }
+}
 
-/** One orbit per lane, driven as a state machine around ONE call of the right-hand side per
-    loop iteration: lanes of a warp at different stages, attempts, orbits or in the initial-step
-    estimate all meet at that call, instead of serialising at twelve separate call sites.  The
-    step algorithm (OdeStepperDOP853::initTimeStep / doStep and the run loop of
-    BaseOrbitIntegrator::run, src/math_ode.cpp:35-406, src/orbit.cpp:52-84) is unchanged:
+/// phases of a lane: without an orbit, beginning one (the three evaluations of the initial-step
+/// estimate) or in the stages of an attempt
+enum { PH_IDLE, PH_INIT, PH_STAGE };
+
+/** One orbit per lane.  The lanes of a warp go through the twelve right-hand sides of an attempt
+    together: all are at the same row of the Runge-Kutta table, so the row is a branch that the whole
+    warp takes, with the row's own terms, constants and stage slots written out, around one (inlined)
+    evaluation of the right-hand side.  A lane whose attempt is accepted or rejected begins its next
+    one in the same breath; a lane whose orbit ends takes another from the queue and makes its three
+    initial evaluations during the last three rows of the others' next attempt (of ~500 attempts an
+    orbit that one is lost).  What bounds a batch is the serial chain of its longest orbits: one orbit
+    alone took 120-175 ms of the 166-245 ms of 1e4 triaxial or 3e3 bar orbits, 3000-3500 instructions
+    per evaluation, most of them not arithmetic (per-lane rows with nine table-driven terms, the
+    selection of the harmonics' cosines by comparing every order with every slot, the asymptotic
+    expansions' coefficient loops).
+
+    The step algorithm (OdeStepperDOP853::initTimeStep / doStep and the run loop of
+    BaseOrbitIntegrator::run, src/math_ode.cpp:35-406, src/orbit.cpp:52-84):
     initial step from Euler and Heun probes, error norm err5 |h| / sqrt(6 (err5 + 0.01 err3))
     weighted by (accAbs + accRel max|x|) accFac, accept at err <= 1, step factor
     min(finc, safe / err^(1/8)), rejection with the nbad counter; the final point is rotated
@@ -182,46 +215,42 @@ enum { PH_FETCH, PH_INIT1, PH_INIT2, PH_INIT3, PH_STAGE, PH_FINISH };
     queue != nullptr: lanes take orbits from the work counter until it passes n; otherwise lane
     i integrates orbit i only.
     G > 1: a group of G consecutive lanes integrates one orbit: every lane of the group runs the
-    same state machine on the same data (the group's sums are bit-identical in all its lanes, so
+    same integration on the same data (the group's sums are bit-identical in all its lanes, so
     its control flow never splits) and the lanes share the spline evaluations of each right-hand
     side; lane 0 of the group takes the orbits from the counter and writes the results.
     MIXED: the forces of the multi-harmonic kind with the m != 0 harmonics in FP32 (the radial m = 0
     part, the Fourier sums, the state, the stages and the error norm stay FP64). */
 template<int KIND, int G, bool MIXED>
-__global__ void __launch_bounds__(ORBIT_BLOCK_MAX) dop853Kernel(const __grid_constant__ MultipoleView M, const OrbitParams P,
-    long n, const double* __restrict__ ic, const double* __restrict__ T, double* __restrict__ out,
-    long* __restrict__ nsteps, long* __restrict__ nrej, int* __restrict__ status,
+__global__ void __launch_bounds__(ORBIT_BLOCK_MAX) dop853Kernel(const __grid_constant__ MultipoleView M,
+    const __grid_constant__ OrbitParams P, long n, const double* __restrict__ ic, const double* __restrict__ T,
+    double* __restrict__ out, long* __restrict__ nsteps, long* __restrict__ nrej, int* __restrict__ status,
     unsigned long long* queue)
 {
     const int gl = threadIdx.x % G;
     const unsigned gmask = groupMask<G>();
     using namespace dp853;
     extern __shared__ double smem[];
-    __shared__ StageTable tab;
-    for(int k = threadIdx.x; k < static_cast<int>(sizeof(StageTable) / sizeof(double)); k += blockDim.x)
-        reinterpret_cast<double*>(&tab)[k] = reinterpret_cast<const double*>(&STAGE_TABLE)[k];
-    __syncthreads();
     const StageStore S{ smem + threadIdx.x, static_cast<int>(blockDim.x) };
     const double Om = P.Omega;
 
     long i = queue ? -1 : (blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x) / G;
-    if(!queue && i >= n) return;
-    int phase = queue ? PH_FETCH : PH_INIT1;
-    double x[6], k1[6], xt[6], k1b[6];
+    bool drained = !queue && i >= n, first = true;      // no orbit left; no orbit taken yet
+    int phase = PH_IDLE;
+    double x[6], k1[6], xt[6], acc[6];
     double t = 0, tEnd = 0, sign = 1, h = 0, h1 = 0, hNext = 0, accFac = 1, preverr = INFINITY, tb = 0, hLast = 0,
         remaining = 0, targetTime = 0;
     long steps = 0, rejects = 0;
-    int st = ORBIT_OK, row = 0, nbad = 0, attempts = 0;
+    int st = ORBIT_OK, nbad = 0, attempts = 0;
+    bool finished = false;
 
     // begin an attempt with the current h (zero, non-finite or endlessly rejected: give up)
     auto startAttempt = [&]() {
-        if(h == 0 || !isFinite(h) || ++attempts > MAX_ATTEMPTS_PER_STEP) { st = ORBIT_BAD_STEP; phase = PH_FINISH; return; }
-        row = 0;
+        if(h == 0 || !isFinite(h) || ++attempts > MAX_ATTEMPTS_PER_STEP) { st = ORBIT_BAD_STEP; finished = true; return; }
         phase = PH_STAGE;
     };
     // begin the next step, or finish the orbit when the end time is reached
     auto startStep = [&]() {
-        if(t == tEnd) { phase = PH_FINISH; return; }
+        if(t == tEnd) { finished = true; return; }
         remaining = tEnd - t;
         h = fmin(remaining * sign, hNext) * sign;
         nbad = 0; attempts = 0; preverr = INFINITY;
@@ -229,38 +258,162 @@ __global__ void __launch_bounds__(ORBIT_BLOCK_MAX) dop853Kernel(const __grid_con
     };
 
     while(true) {
-        if(phase == PH_FETCH) {
-            long v = 0;
-            if(gl == 0) v = static_cast<long>(atomicAdd(queue, 1ull));
-            i = G > 1 ? static_cast<long>(__shfl_sync(gmask, static_cast<unsigned long long>(v), 0, G)) : v;
-            if(i >= n) break;
-            phase = PH_INIT1;
-        }
-        if(phase == PH_INIT1) {          // a new orbit: load its start
-            for(int c = 0; c < 6; c++) x[c] = ic[6 * i + c];
-            tEnd = T[i];
-            t = 0; tb = 0; hLast = 0; steps = 0; rejects = 0; st = ORBIT_OK; accFac = 1; targetTime = 0;
-            sign = tEnd >= 0 ? 1 : -1;
-            if(P.traj && gl == 0) {
-                // no sample yet; an orbit that is not integrated gets its start as sample 0 (and, for
-                // T = 0, as sample 1 too: the reference's zero sampling interval records the start
-                // and the end of its single zero step)
-                double* o = P.traj + i * P.trajSize * 6;
-                for(int k = 0; k < P.trajSize * 6; k++) o[k] = NAN;
-                if(tEnd == 0 || !isFinite(tEnd))
-                    for(int k = 0; k < (tEnd == 0 ? 2 : 1) && k < P.trajSize; k++)
-                        for(int c = 0; c < 6; c++) o[6 * k + c] = x[c];
+        // ---- lanes without an orbit take one
+        if(phase == PH_IDLE && !drained) {
+            if(queue) {
+                long v = 0;
+                if(gl == 0) v = static_cast<long>(atomicAdd(queue, 1ull));
+                i = G > 1 ? static_cast<long>(__shfl_sync(gmask, static_cast<unsigned long long>(v), 0, G)) : v;
+                drained = i >= n;
+            } else
+                drained = !first;
+            first = false;
+            if(!drained) {
+                for(int c = 0; c < 6; c++) x[c] = ic[6 * i + c];
+                tEnd = T[i];
+                t = 0; tb = 0; hLast = 0; steps = 0; rejects = 0; st = ORBIT_OK; accFac = 1; targetTime = 0;
+                sign = tEnd >= 0 ? 1 : -1;
+                finished = false;
+                phase = PH_INIT;
+                if(P.traj && gl == 0) {
+                    // no sample yet; an orbit that is not integrated gets its start as sample 0 (and, for
+                    // T = 0, as sample 1 too: the reference's zero sampling interval records the start
+                    // and the end of its single zero step)
+                    double* o = P.traj + i * P.trajSize * 6;
+                    for(int k = 0; k < P.trajSize * 6; k++) o[k] = NAN;
+                    if(tEnd == 0 || !isFinite(tEnd))
+                        for(int k = 0; k < (tEnd == 0 ? 2 : 1) && k < P.trajSize; k++)
+                            for(int c = 0; c < 6; c++) o[6 * k + c] = x[c];
+                }
             }
         }
-        if(phase == PH_FINISH) {
+        if(!__any_sync(FULL_MASK, phase != PH_IDLE)) break;
+        // ---- the rows of an attempt, from the first one that a lane of the warp needs
+        for(int row = __any_sync(FULL_MASK, phase == PH_STAGE) ? 0 : INIT_ROW; row < NUM_ROWS; row++) {
+            double tt = t;
+            if(phase == PH_STAGE) {
+                switch(row) {
+                    case 0:  stagePoint<0>(S, x, k1, h, acc, xt); break;
+                    case 1:  stagePoint<1>(S, x, k1, h, acc, xt); break;
+                    case 2:  stagePoint<2>(S, x, k1, h, acc, xt); break;
+                    case 3:  stagePoint<3>(S, x, k1, h, acc, xt); break;
+                    case 4:  stagePoint<4>(S, x, k1, h, acc, xt); break;
+                    case 5:  stagePoint<5>(S, x, k1, h, acc, xt); break;
+                    case 6:  stagePoint<6>(S, x, k1, h, acc, xt); break;
+                    case 7:  stagePoint<7>(S, x, k1, h, acc, xt); break;
+                    case 8:  stagePoint<8>(S, x, k1, h, acc, xt); break;
+                    case 9:  stagePoint<9>(S, x, k1, h, acc, xt); break;
+                    case 10: stagePoint<10>(S, x, k1, h, acc, xt); break;
+                    default: stagePoint<11>(S, x, k1, h, acc, xt);
+                }
+                tt = t + STAGE_TABLE.c[row] * h;     // c = 1 for k12 and the 8th-order point: t + h
+            } else if(phase == PH_INIT && row == INIT_ROW) {
+                for(int c = 0; c < 6; c++) xt[c] = x[c];
+            } else if(phase == PH_INIT && row == INIT_ROW + 1) {
+                tt = t + h1;
+                for(int c = 0; c < 6; c++) xt[c] = x[c] + h1 * k1[c];
+            } else if(phase == PH_INIT && row == INIT_ROW + 2) {
+                tt = t + h1;
+                for(int c = 0; c < 6; c++) xt[c] = x[c] + 0.5 * h1 * (k1[c] + S.at(0, c));
+            }
+            // ---- the one evaluation site
+            if(phase == PH_STAGE || (phase == PH_INIT && row >= INIT_ROW && !finished)) {
+                double k[6];
+                const bool wantAcc = phase == PH_INIT ? row == INIT_ROW : row == NUM_ROWS - 1;
+                double af = 1;
+                orbitRHS<KIND, G, MIXED>(M, Om, tt, xt, k, wantAcc ? &af : nullptr);
+                if(phase == PH_STAGE) {
+                    if(row < NUM_ROWS - 1) {
+                        const int d = row < 9 ? row : row - 9;          // k11, k12 take the places of k2, k3
+                        for(int c = 0; c < 6; c++) S.at(d, c) = k[c];
+                    } else {
+                        // ---- error estimate (3rd and 5th order embedded solutions), k13 = k, acc = k1 of b
+                        double err5 = 0, err3 = 0;
+                        for(int c = 0; c < 6; c++) {
+                            const double sk = (P.accAbs + P.accRel * fmax(fabs(x[c]), fabs(xt[c]))) * af;
+                            if(sk == 0) continue;
+                            err3 += pow2((acc[c] - bhh1 * k1[c] - bhh2 * S.at(7, c) - bhh3 * S.at(1, c)) / sk);
+                            err5 += pow2((sumProducts(er1, k1[c], er6, S.at(4, c)) + er7 * S.at(5, c) + er8 * S.at(6, c) +
+                                er9 * S.at(7, c) + er10 * S.at(8, c) + er11 * S.at(0, c) + er12 * S.at(1, c)) / sk);
+                        }
+                        const double den = sqrt(6 * (err5 + 0.01 * err3));
+                        const double err = den == 0 ? 0 : err5 * fabs(h) / den;
+                        if(!isFinite(err)) { st = ORBIT_NONFINITE; finished = true; }
+                        else {
+                            double fac = sqrt(sqrt(sqrt(err)));
+                            bool accepted = false;
+                            if(err <= 1) {
+                                hNext = fabs(h) * fmin(finc, safe / fac);
+                                accepted = true;
+                            } else {
+                                if(err > 0.5 * preverr) {
+                                    nbad++;
+                                    if(nbad >= 2) fac = 1 / fdec;
+                                    if(nbad >= 4) { hNext = fabs(h); accepted = true; }
+                                } else
+                                    nbad = 0;
+                                if(!accepted) {
+                                    preverr = err;
+                                    h *= fmax(fdec, safe / fac);
+                                    rejects++;
+                                    startAttempt();
+                                }
+                            }
+                            if(accepted) {
+                                if(P.traj && gl == 0) sampleStep(P, i, tEnd, sign, t, h, x, xt, k1, k, S);
+                                if(P.target.degree >= 0 && gl == 0) {
+                                    targetStep(P, i, t, h, x, xt, k1, k, S);
+                                    targetTime += h;
+                                }
+                                for(int c = 0; c < 6; c++) { x[c] = xt[c]; k1[c] = k[c]; }
+                                tb = t;
+                                hLast = h;
+                                t = h == remaining ? tEnd : t + h;
+                                if(++steps >= P.maxSteps) {
+                                    if(t != tEnd) st = ORBIT_MAX_STEPS;
+                                    finished = true;
+                                } else
+                                    startStep();
+                            }
+                        }
+                    }
+                } else if(row == INIT_ROW) {
+                    for(int c = 0; c < 6; c++) k1[c] = k[c];
+                    accFac = af;
+                    if(tEnd == 0 || !isFinite(tEnd)) finished = true;
+                    else {
+                        double nx = 0, nd = 0;
+                        for(int c = 0; c < 6; c++) { nx += x[c] * x[c]; nd += k1[c] * k1[c]; }
+                        h1 = fmax(HMIN, fmin(HMAX, sqrt(nx / nd) * 0.01));
+                    }
+                } else if(row == INIT_ROW + 1) {
+                    for(int c = 0; c < 6; c++) S.at(0, c) = k[c];
+                } else {
+                    // initTimeStep (src/math_ode.cpp:35-91): Euler + Heun probes, Aarseth-like estimate
+                    double h2 = INFINITY;
+                    for(int c = 0; c < 6; c++) {
+                        const double k2c = S.at(0, c);
+                        const double d0 = fmax(P.accAbs, fmax(fabs(x[c]), fabs(xt[c])));
+                        const double d1 = fmax(fabs(k1[c]), fabs(k[c]));
+                        const double d2 = fabs((3 * k2c - k1[c] - 2 * k[c]) / h1);
+                        const double d3 = fabs(6 * (k[c] - k2c) / (h1 * h1));
+                        h2 = fmin(h2, sumProducts(d1, d1, d0, d2) / sumProducts(d2, d2, d1, d3));
+                    }
+                    hNext = fmax(HMIN, fmin(HMAX, pow(P.accRel, 1. / 8) * sqrt(h2))) * accFac;
+                    startStep();
+                }
+            }
+        }
+        // ---- results of the orbits that ended
+        if(finished && phase != PH_IDLE) {
             if(gl == 0) {
                 double ca = 1, sa = 0;
                 if(Om != 0) sincos(Om * (hLast + tb), &sa, &ca);
-                out[6 * i + 0] = x[0] * ca + x[1] * sa;
-                out[6 * i + 1] = x[1] * ca - x[0] * sa;
+                out[6 * i + 0] = sumProducts(x[0], ca, x[1], sa);
+                out[6 * i + 1] = sumProducts(x[1], ca, -x[0], sa);
                 out[6 * i + 2] = x[2];
-                out[6 * i + 3] = x[3] * ca + x[4] * sa;
-                out[6 * i + 4] = x[4] * ca - x[3] * sa;
+                out[6 * i + 3] = sumProducts(x[3], ca, x[4], sa);
+                out[6 * i + 4] = sumProducts(x[4], ca, -x[3], sa);
                 out[6 * i + 5] = x[5];
                 if(nsteps) nsteps[i] = steps;
                 if(nrej) nrej[i] = rejects;
@@ -277,114 +430,8 @@ __global__ void __launch_bounds__(ORBIT_BLOCK_MAX) dop853Kernel(const __grid_con
                     }
                 }
             }
-            if(!queue) break;
-            phase = PH_FETCH;
-            continue;
-        }
-        // ---- the point at which the right-hand side is wanted
-        double tt;
-        if(phase == PH_INIT1) {
-            tt = t;
-            for(int c = 0; c < 6; c++) xt[c] = x[c];
-        } else if(phase == PH_INIT2) {
-            tt = t + h1;
-            for(int c = 0; c < 6; c++) xt[c] = x[c] + h1 * k1[c];
-        } else if(phase == PH_INIT3) {
-            tt = t + h1;
-            for(int c = 0; c < 6; c++) xt[c] = x[c] + 0.5 * h1 * (k1[c] + S.at(0, c));
-        } else {
-            tt = t + tab.c[row] * h;     // c = 1 for k12 and the 8th-order point: t + h
-            for(int c = 0; c < 6; c++) {
-                double acc = tab.coef[row][0] * k1[c];
-                for(int m = 1; m < MAX_TERMS; m++) {
-                    const int sl = tab.src[row][m];
-                    acc += tab.coef[row][m] * (sl < 0 ? k1[c] : S.at(sl, c));
-                }
-                if(row == NUM_ROWS - 1) k1b[c] = acc;
-                xt[c] = x[c] + h * acc;
-            }
-        }
-        // ---- the one evaluation site
-        const bool wantAcc = phase == PH_INIT1 || (phase == PH_STAGE && row == NUM_ROWS - 1);
-        double k[6], af = 1;
-        orbitRHS<3, KIND, G, MIXED>(M, Om, tt, xt, k, wantAcc ? &af : nullptr);
-        // ---- use the result
-        if(phase == PH_INIT1) {
-            for(int c = 0; c < 6; c++) k1[c] = k[c];
-            accFac = af;
-            if(tEnd == 0 || !isFinite(tEnd)) { phase = PH_FINISH; continue; }
-            double nx = 0, nd = 0;
-            for(int c = 0; c < 6; c++) { nx += x[c] * x[c]; nd += k1[c] * k1[c]; }
-            h1 = fmax(HMIN, fmin(HMAX, sqrt(nx / nd) * 0.01));
-            phase = PH_INIT2;
-        } else if(phase == PH_INIT2) {
-            for(int c = 0; c < 6; c++) S.at(0, c) = k[c];
-            phase = PH_INIT3;
-        } else if(phase == PH_INIT3) {
-            // initTimeStep (src/math_ode.cpp:35-91): Euler + Heun probes, Aarseth-like estimate
-            double h2 = INFINITY;
-            for(int c = 0; c < 6; c++) {
-                const double k2c = S.at(0, c);
-                const double d0 = fmax(P.accAbs, fmax(fabs(x[c]), fabs(xt[c])));
-                const double d1 = fmax(fabs(k1[c]), fabs(k[c]));
-                const double d2 = fabs((3 * k2c - k1[c] - 2 * k[c]) / h1);
-                const double d3 = fabs(6 * (k[c] - k2c) / (h1 * h1));
-                h2 = fmin(h2, (d0 * d2 + d1 * d1) / (d1 * d3 + d2 * d2));
-            }
-            hNext = fmax(HMIN, fmin(HMAX, pow(P.accRel, 1. / 8) * sqrt(h2))) * accFac;
-            startStep();
-        } else if(row < NUM_ROWS - 1) {
-            const int d = tab.dest[row];
-            for(int c = 0; c < 6; c++) S.at(d, c) = k[c];
-            row++;
-        } else {
-            // ---- error estimate (3rd and 5th order embedded solutions), k13 = k
-            double err5 = 0, err3 = 0;
-            for(int c = 0; c < 6; c++) {
-                const double sk = (P.accAbs + P.accRel * fmax(fabs(x[c]), fabs(xt[c]))) * af;
-                if(sk == 0) continue;
-                err3 += pow2((k1b[c] - bhh1 * k1[c] - bhh2 * S.at(7, c) - bhh3 * S.at(1, c)) / sk);
-                err5 += pow2((er1 * k1[c] + er6 * S.at(4, c) + er7 * S.at(5, c) + er8 * S.at(6, c) +
-                    er9 * S.at(7, c) + er10 * S.at(8, c) + er11 * S.at(0, c) + er12 * S.at(1, c)) / sk);
-            }
-            const double den = sqrt(6 * (err5 + 0.01 * err3));
-            const double err = den == 0 ? 0 : err5 * fabs(h) / den;
-            if(!isFinite(err)) { st = ORBIT_NONFINITE; phase = PH_FINISH; continue; }
-            double fac = sqrt(sqrt(sqrt(err)));
-            bool accepted = false;
-            if(err <= 1) {
-                hNext = fabs(h) * fmin(finc, safe / fac);
-                accepted = true;
-            } else {
-                if(err > 0.5 * preverr) {
-                    nbad++;
-                    if(nbad >= 2) fac = 1 / fdec;
-                    if(nbad >= 4) { hNext = fabs(h); accepted = true; }
-                } else
-                    nbad = 0;
-                if(!accepted) {
-                    preverr = err;
-                    h *= fmax(fdec, safe / fac);
-                    rejects++;
-                    startAttempt();
-                    continue;
-                }
-            }
-            if(P.traj && gl == 0) sampleStep(P, i, tEnd, sign, t, h, x, xt, k1, k, S);
-            if(P.target.degree >= 0 && gl == 0) {
-                targetStep(P, i, t, h, x, xt, k1, k, S);
-                targetTime += h;
-            }
-            for(int c = 0; c < 6; c++) { x[c] = xt[c]; k1[c] = k[c]; }
-            tb = t;
-            hLast = h;
-            t = h == remaining ? tEnd : t + h;
-            if(++steps >= P.maxSteps) {
-                if(t != tEnd) st = ORBIT_MAX_STEPS;
-                phase = PH_FINISH;
-                continue;
-            }
-            startStep();
+            phase = PH_IDLE;
+            finished = false;
         }
     }
 }

@@ -187,6 +187,12 @@ DevicePotential* createDevicePotential(const std::vector<double>& radii,
         V.inner.S = P->innerS.ptr; V.inner.U = P->innerU.ptr; V.inner.W = P->innerW.ptr;
         V.outer.ind = H.outer.ind; V.outer.r0sq = H.outer.r0sq; V.outer.inner = 0; V.outer.Q = H.outer.Q;
         V.outer.S = P->outerS.ptr; V.outer.U = P->outerU.ptr; V.outer.W = P->outerW.ptr;
+        std::vector<double> norm((LMAX_MAX + 1) * (LMAX_MAX + 1), 1.);
+        for(int m = 0; m <= LMAX_MAX; m++)
+            for(int l = m + 1; l <= LMAX_MAX; l++)
+                norm[m * (LMAX_MAX + 1) + l] = sqrt((2 * l + 1.) / (2 * l - 1.) * (l - m) / (l + m));
+        P->legendreNorm.upload(norm);
+        V.inner.norm = V.outer.norm = P->legendreNorm.ptr;
         P->axisymmetric = (H.ind.sym & SYM_AXISYMMETRIC) == SYM_AXISYMMETRIC;
         // register-resident evaluator: m = 0 first, then ascending m
         V.nFast = 0;
