@@ -1,5 +1,5 @@
 // DOP853 orbit integration on the device: one orbit per thread, Runge-Kutta stage vectors in
-// shared memory (thread-interleaved, bank-conflict free), state and step control in registers.
+// shared memory, state and step control in registers.
 #pragma once
 #include "multipole_force.cuh"
 

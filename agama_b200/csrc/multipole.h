@@ -78,6 +78,12 @@ struct MultipoleView {
     /// s^i t^j (j fastest) with s, t the position in the cell in units of its widths, from the
     /// lower ln r node and from the tau node nearer the pole; null where there are none (nFast = 0)
     const double* cells;
+    /// the same cells for the node form (orbits), [slot][nr-1][nt-1][CELL_COEFS]: for each of the six
+    /// functions whose segments in tau are taken first (f, f_x, f_xx at the lower and upper ln r node:
+    /// f, f, fx, fx, fxx, fxx) the value and two tau derivatives at the lower tau node and the three
+    /// defects at the upper one (quinticSegment); f relative to the corner (xlow, ylow), whose own
+    /// value stands in the first place (where the difference would be 0)
+    const double* segments;
     const float* spl2d32; // the same table rounded to FP32 (mixed-precision evaluation of m != 0)
     const double* spl1d;  // [c][nr][3]: f f' f''  (1-D case; all (lmax+1)^2 coefficients)
     int logScaling;

@@ -15,33 +15,142 @@ namespace agb {
 /// a b + c d with c d rounded
 __device__ __forceinline__ double sumProducts(double a, double b, double c, double d) { return fma(a, b, __dmul_rn(c, d)); }
 
+/// a / b correctly rounded from y = 1 / b correctly rounded (Markstein 1990: a quotient estimate within
+/// one unit in the last place, its exact remainder by a fused multiply-add, and y give the rounded
+/// quotient; the first step brings a y to such an estimate).  For a and b well inside the range of
+/// normal numbers, a = 0 included.
+__device__ __forceinline__ double quotient(double a, double b, double y)
+{
+    const double q0 = a * y, q1 = fma(fma(-b, q0, a), y, q0);
+    return fma(fma(-b, q1, a), y, q1);
+}
+
+/// 1 / b correctly rounded, for b well inside the range of normal numbers (the same step)
+__device__ __forceinline__ double reciprocal(double b)
+{
+    const double y = rcpNormal(b);
+    return fma(fma(-b, y, 1.0), y, y);
+}
+
+/// sqrt(a) correctly rounded, for a > 0 well inside the range of normal numbers: the root estimate a y
+/// corrected by its exact remainder (Markstein)
+__device__ __forceinline__ double squareRoot(double a)
+{
+    const double y = rsqrtNormal(a), g = a * y;
+    return fma(fma(-g, g, a), 0.5 * y, g);
+}
+
+/// the basis of a quintic segment at one point (quinticSegmentR): f = fl + bf d0 + dx f1l + b1 d1 + e f2l + b2 d2,
+/// f' = bfp d0 + f1l + b1p d1 + dx f2l + b2p d2
+struct SegmentBasis {
+    double bf, dx, b1, e, b2, bfp, b1p, b2p;
+    __device__ __forceinline__ SegmentBasis(double x, double xl, double xh, double hi)
+    {
+        dx = x - xl;
+        const double h = xh - xl, h2 = h * h, t = dx * hi, t2 = t * t, t3 = t * t2, omt = t * (1 - t);
+        e = 0.5 * dx * dx;
+        bf = t3 * (10 - t * (15 - 6 * t));
+        b1 = t3 * (1 - t * 0.5) * h;
+        b2 = t3 * (1 - t * (1.25 - 0.5 * t)) * h2;
+        bfp = 30 * omt * hi * omt;
+        b1p = t2 * (3 - t * 2);
+        b2p = t2 * (3 - t * (5 - 2.5 * t)) * h;
+    }
+    __device__ __forceinline__ double value(double fl, double f1l, double f2l, double d0, double d1, double d2) const
+    {
+        return fma(b2, d2, fma(e, f2l, fma(b1, d1, fma(dx, f1l, fma(bf, d0, fl)))));
+    }
+    __device__ __forceinline__ double slope(double f1l, double f2l, double d0, double d1, double d2) const
+    {
+        return fma(b2p, d2, fma(dx, f2l, fma(b1p, d1, fma(bfp, d0, f1l))));
+    }
+};
+
+/** spline2dCell for value and gradient away from the upper nodes of a cell, from its segments in the
+    second direction (MultipoleView::segments): what depends on the table alone -- the three defects of
+    each segment, a quarter of the arithmetic -- is tabulated, by the same operations.
+    (y: the basis in tau, x: in ln r, hx: the width of the cell in ln r) */
+__device__ __forceinline__ void segmentCell(const double* __restrict__ c, const SegmentBasis& x, double hx,
+    const SegmentBasis& y, double* z, double* zx, double* zy)
+{
+    double F[6], G[6], off = 0;
+#pragma unroll
+    for(int p = 0; p < 6; p += 2) {
+        double w[12];
+        ldg4(c + 6 * p, w);
+        ldg4(c + 6 * p + 4, w + 4);
+        ldg4(c + 6 * p + 8, w + 8);
+        if(p == 0) { off = w[0]; w[0] = 0; }
+#pragma unroll
+        for(int a = 0; a < 2; a++) {
+            const double* s = w + 6 * a;
+            F[p + a] = y.value(s[0], s[1], s[2], s[3], s[4], s[5]);
+            G[p + a] = y.slope(s[1], s[2], s[3], s[4], s[5]);
+        }
+    }
+    auto defects = [&](const double* f, double* d) {
+        d[0] = fma(-(0.5 * hx), f[3] + f[2], f[1] - f[0]);
+        d[1] = fma(-(0.5 * hx), f[5] + f[4], f[3] - f[2]);
+        d[2] = f[5] - f[4];
+    };
+    double d[3];
+    defects(F, d);
+    *z = x.value(F[0], F[2], F[4], d[0], d[1], d[2]) + off;
+    *zx = x.slope(F[2], F[4], d[0], d[1], d[2]);
+    defects(G, d);
+    *zy = x.value(G[0], G[2], G[4], d[0], d[1], d[2]);
+}
+
 /** evalInterp2dFast for value and gradient with the harmonics taken one after the other: each one is
     evaluated, scaled and added to the Fourier sums (m = 0 first, then by ascending m), and the
     cosine and sine of m phi follow by the same multiple-angle recurrence up to |m| (begun anew where |m|
     falls), so nothing is kept per harmonic.
     G > 1: the lanes of a group take G harmonics at a time, one each, and every lane adds all of them
     in the same order from the lane that evaluated it, so every G gives the same bits.
-    MIXED: the m != 0 harmonics from the FP32 table. */
+    MIXED: the m != 0 harmonics from the FP32 table.
+    NODES: the cells from the node values, for points at an upper node of either direction (the last
+    ones of the grids, where the node values are taken without round-off). */
+template<int KIND, int G, bool MIXED, bool NODES>
+__device__ __forceinline__ void forceInterp2d(const MultipoleView& M, double R, double z, double phi, double* pot,
+    CylDerivs* g);
+
 template<int KIND, int G, bool MIXED>
+__device__ __noinline__ void forceAtUpperNode(const MultipoleView& M, double R, double z, double phi, double* pot,
+    CylDerivs* g)
+{
+    forceInterp2d<KIND, G, MIXED, true>(M, R, z, phi, pot, g);
+}
+
+template<int KIND, int G, bool MIXED, bool NODES>
 __device__ __forceinline__ void forceInterp2d(const MultipoleView& M, double R, double z, double phi, double* pot,
     CylDerivs* g)
 {
     const int gl = G > 1 ? static_cast<int>(threadIdx.x % G) : 0;
     const unsigned gmask = G > 1 ? groupMask<G>() : 0u;
-    const double r = sqrt(sumProducts(z, z, R, R)), logr = log(r), rpRinv = 1. / (r + fabs(R));
+    const double r = squareRoot(sumProducts(z, z, R, R)), logr = log(r), rpRinv = reciprocal(r + fabs(R));
     const double tau = R == 0 ? signOf(z) : z * rpRinv;
     const bool inside = logr >= M.gridR.x0 && logr <= M.gridR.xEnd && tau >= M.gridTau.x0 && tau <= M.gridTau.xEnd;
     double xl, xh, yl, yh, xhi, yhi;
     const int xs = gridCell(M.gridR, logr, &xl, &xh, &xhi), ys = gridCell(M.gridTau, tau, &yl, &yh, &yhi);
+    if(!NODES && (logr == xh || tau == yh)) {
+        forceAtUpperNode<KIND, G, MIXED>(M, R, z, phi, pot, g);
+        return;
+    }
+    const SegmentBasis bx(logr, xl, xh, xhi), by(tau, yl, yh, yhi);
     const size_t slotStride = static_cast<size_t>(M.nr) * M.nt * NODE_STRIDE;
+    const size_t segmentStride = static_cast<size_t>(M.nr - 1) * (M.nt - 1) * CELL_COEFS;
+    const double* segments = M.segments + (static_cast<size_t>(xs) * (M.nt - 1) + ys) * CELL_COEFS;
     auto cell = [&](int s, double* P, double* Dr, double* Dt) {
+        const int slot = M.fastSlot[s];
         double rr, rt, tt;
         if(MIXED && s > 0)      // m != 0 (angular) harmonics in FP32, the radial m = 0 one in FP64
-            spline2dCell32<3>(M.spl2d32 + M.fastSlot[s] * slotStride, M.nt, xs, ys, logr, xl, xh, tau, yl, yh,
+            spline2dCell32<3>(M.spl2d32 + slot * slotStride, M.nt, xs, ys, logr, xl, xh, tau, yl, yh,
+                P, Dr, Dt, &rr, &rt, &tt);
+        else if(NODES)
+            spline2dCell<3>(M.spl2d + slot * slotStride, M.nt, xs, ys, logr, xl, xh, tau, yl, yh, xhi, yhi,
                 P, Dr, Dt, &rr, &rt, &tt);
         else
-            spline2dCell<3>(M.spl2d + M.fastSlot[s] * slotStride, M.nt, xs, ys, logr, xl, xh, tau, yl, yh,
-                xhi, yhi, P, Dr, Dt, &rr, &rt, &tt);
+            segmentCell(segments + slot * segmentStride, bx, xh - xl, by, P, Dr, Dt);
         if(!inside) *P = *Dr = *Dt = NAN;
     };
     const int numHarm = KIND == EVAL_AXI ? 1 : M.nFast;
@@ -65,7 +174,7 @@ __device__ __forceinline__ void forceInterp2d(const MultipoleView& M, double R, 
                 P0 = __shfl_sync(gmask, P0, 0, G); Dr0 = __shfl_sync(gmask, Dr0, 0, G); Dt0 = __shfl_sync(gmask, Dt0, 0, G);
             }
             if(M.logScaling) {
-                const double ex = exp(P0), val = 1 / (M.invPhi0 - ex);
+                const double ex = exp(P0), val = reciprocal(M.invPhi0 - ex);
                 P0 = val;
                 const double dPdX = val * val * ex;
                 Dr0 *= dPdX;
@@ -105,21 +214,11 @@ __device__ __forceinline__ void forceInterp2d(const MultipoleView& M, double R, 
             }
         }
     }
-    const double rinv = 1 / r, r2inv = rinv * rinv;
+    const double rinv = reciprocal(r), r2inv = rinv * rinv;
     const double drdR = R * r2inv, drdz = z * r2inv, dtdR = -tau * rinv, dtdz = rinv - rpRinv;
     g->dR = sumProducts(gs.dr, drdR, gs.dt, dtdR);
     g->dz = sumProducts(gs.dr, drdz, gs.dt, dtdz);
     g->dphi = gs.dphi;
-}
-
-/// a / b correctly rounded from y = 1 / b correctly rounded (Markstein 1990: a quotient estimate within
-/// one unit in the last place, its exact remainder by a fused multiply-add, and y give the rounded
-/// quotient; the first step brings a y to such an estimate).  For a and b well inside the range of
-/// normal numbers, a = 0 included.
-__device__ __forceinline__ double quotient(double a, double b, double y)
-{
-    const double q0 = a * y, q1 = fma(fma(-b, q0, a), y, q0);
-    return fma(fma(-b, q1, a), y, q1);
 }
 
 /** evalPowerLaw for value and gradient and expansions with cosine terms only (lmax > 2 or one harmonic):
@@ -245,16 +344,17 @@ __device__ __forceinline__ void powerLawTerms(const PowerLawView& A, double R, d
 /// beyond the 2-D splines: asymptotic expansions (and 1-D splines); out of line
 static __device__ __noinline__ void forceBeyond(const MultipoleView& M, double R, double z, double phi, double* pot, CylDerivs* g)
 {
-    // (the caller's rsq: a 2-D potential comes here only from beyond its grid)
     const double rsq = sumProducts(R, R, z, z);
     CylHess h;
-    if(M.is2d || rsq < M.rInnerSq || rsq > M.rOuterSq) {
+    if(rsq < M.rInnerSq || rsq > M.rOuterSq) {
         const PowerLawView& A = rsq < M.rInnerSq ? M.inner : M.outer;
         if(A.ind.mmin() == 0 && (A.ind.lmax != 2 || A.ind.step != 2))
             powerLawTerms(A, R, z, phi, pot, g);
         else
             evalPowerLaw<3>(A, R, z, phi, pot, g, &h);
-    } else
+    } else if(M.is2d)
+        evalInterp2d<3>(M, R, z, phi, pot, g, &h);      // (2-D splines without cells)
+    else
         evalInterp1d<3>(M, R, z, phi, pot, g, &h);
 }
 
@@ -262,7 +362,10 @@ static __device__ __noinline__ void forceBeyond(const MultipoleView& M, double R
 template<int KIND, int G, bool MIXED>
 __device__ __forceinline__ void evalForceCar(const MultipoleView& M, double x, double y, double z, double* pot, double* grad)
 {
-    const double R = sqrt(sumProducts(x, x, y, y));
+    // (squares that leave the range of normal numbers take the library's root and divisions)
+    const double R2 = sumProducts(x, x, y, y);
+    const bool usual = R2 > 1e-200 && R2 < 1e200;
+    const double R = usual ? squareRoot(R2) : sqrt(R2);
     // a potential with only m = 0 terms (its splines and both asymptotes): its evaluators neither
     // read the azimuth nor give a phi derivative (exactly 0), so neither atan2 nor the azimuth's
     // derivatives are formed (the results are the same bits)
@@ -272,9 +375,13 @@ __device__ __forceinline__ void evalForceCar(const MultipoleView& M, double x, d
     if(R == 0) {
         phi = 0; dRdx = dRdy = dphidx = dphidy = 1;
     } else {
-        const double cphi = x / R, sphi = y / R;
+        const double Rinv = usual ? reciprocal(R) : 0;
+        const double cphi = usual ? quotient(x, R, Rinv) : x / R, sphi = usual ? quotient(y, R, Rinv) : y / R;
         dRdx = cphi; dRdy = sphi;
-        if(!noAzimuth) { dphidx = -sphi / R; dphidy = cphi / R; }
+        if(!noAzimuth) {
+            dphidx = usual ? quotient(-sphi, R, Rinv) : -sphi / R;
+            dphidy = usual ? quotient(cphi, R, Rinv) : cphi / R;
+        }
         phi = noAzimuth ? 0 : atan2(y, x);
     }
     CylDerivs g;
@@ -282,8 +389,8 @@ __device__ __forceinline__ void evalForceCar(const MultipoleView& M, double x, d
     if(KIND == EVAL_GENERAL) {
         CylHess h;
         evalMultipoleCyl<3, KIND>(M, R, z, phi, pot, &g, &h);
-    } else if(!(rsq < M.rInnerSq) && !(rsq > M.rOuterSq) && M.is2d)
-        forceInterp2d<KIND, G, MIXED>(M, R, z, phi, pot, &g);
+    } else if(inCells(M, rsq))
+        forceInterp2d<KIND, G, MIXED, false>(M, R, z, phi, pot, &g);
     else
         forceBeyond(M, R, z, phi, pot, &g);
     grad[0] = noAzimuth ? g.dR * dRdx : sumProducts(g.dR, dRdx, g.dphi, dphidx);

@@ -2,8 +2,7 @@
 //
 // Reference: orbit::BaseOrbitIntegrator::run (src/orbit.cpp:52-84), OrbitIntegrator<Car>::init
 // (:98-117) and OdeStepperDOP853::init / initTimeStep / doStep (src/math_ode.cpp:35-406).
-// Each thread integrates one orbit; the stage vectors k2..k10 live in shared memory laid out
-// [vector][component][thread] so that a warp touches 32 consecutive doubles per access.
+// Each thread integrates one orbit; the stage vectors k2..k10 live in shared memory.
 // A batch is either mapped one orbit per thread, or drained from a device work queue (an
 // atomic counter) by a grid sized to the GPU, which balances orbits of very different length.
 #include "runtime.h"
@@ -27,10 +26,12 @@ constexpr int NUM_STAGE_VECTORS = 9;                 // k2 .. k10 (k11..k13 reus
 constexpr int MAX_ATTEMPTS_PER_STEP = 1000;          // guard against a runaway rejection loop
 constexpr double HMIN = 1e-12, HMAX = 1e12;          // initial-step limits, src/math_ode.cpp:40
 
+/// the stage vectors of one thread: consecutive doubles, so that every access is a constant offset from
+/// one address; an odd number of them per thread keeps the threads of a warp on different banks
+constexpr int STAGE_STRIDE = NUM_STAGE_VECTORS * 6 + 1;
 struct StageStore {
     double* base;
-    int stride;                                      // = blockDim.x
-    __device__ double& at(int v, int c) const { return base[(v * 6 + c) * stride]; }
+    __device__ double& at(int v, int c) const { return base[v * 6 + c]; }
 };
 
 /// The Runge-Kutta stages of one DOP853 attempt as table rows: row r forms the point of stage
@@ -230,7 +231,7 @@ __global__ void __launch_bounds__(ORBIT_BLOCK_MAX) dop853Kernel(const __grid_con
     const unsigned gmask = groupMask<G>();
     using namespace dp853;
     extern __shared__ double smem[];
-    const StageStore S{ smem + threadIdx.x, static_cast<int>(blockDim.x) };
+    const StageStore S{ smem + threadIdx.x * STAGE_STRIDE };
     const double Om = P.Omega;
 
     long i = queue ? -1 : (blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x) / G;
@@ -438,7 +439,7 @@ __global__ void __launch_bounds__(ORBIT_BLOCK_MAX) dop853Kernel(const __grid_con
 
 }  // namespace
 
-size_t orbitSharedBytes(int block) { return sizeof(double) * NUM_STAGE_VECTORS * 6 * block; }
+size_t orbitSharedBytes(int block) { return sizeof(double) * STAGE_STRIDE * block; }
 
 namespace {
 
@@ -463,7 +464,7 @@ OrbitKernel orbitKernel(int kind, int lanes, bool mixed)
 std::atomic<int> g_mixedSetting{ 0 };
 
 /// raise the dynamic shared-memory limit of an orbit kernel on the current device once (the
-/// stage vectors of 128 threads take 54 KB, above the default 48 KB)
+/// stage vectors of 128 threads take 55 KB, above the default 48 KB)
 void allowOrbitSharedMemory(OrbitKernel kernel)
 {
     static std::mutex mutex;

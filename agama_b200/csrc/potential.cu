@@ -104,6 +104,38 @@ __global__ void cellCoefsKernel(int numSlots, int nr, int nt, const GridNode* __
         hermite(G[0][0][j], G[0][1][j], G[0][2][j], G[1][0][j], G[1][1][j], G[1][2][j], c + j, 6);
     c[0] += off;
 }
+
+/// the segments of the 2-D splines cell by cell (MultipoleView::segments): one cell per thread; the
+/// defects by the operations of quinticSegmentR
+__global__ void cellSegmentsKernel(int numSlots, int nr, int nt, const GridNode* __restrict__ gt,
+    const double* __restrict__ nodes, double* __restrict__ segments)
+{
+    const long k = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
+    const long perSlot = static_cast<long>(nr - 1) * (nt - 1);
+    if(k >= numSlots * perSlot) return;
+    const int slot = static_cast<int>(k / perSlot), rem = static_cast<int>(k % perSlot);
+    const int xi = rem / (nt - 1), yi = rem % (nt - 1);
+    const double h = gt[yi + 1].x - gt[yi].x;
+    const double* low = nodes + ((static_cast<size_t>(slot) * nr + xi) * nt + yi) * NODE_STRIDE;
+    const double off = low[0];
+    // node layout: 0 f, 1 fx, 2 fy, 3 fxx, 4 fxy, 5 fyy, 6 fxxy, 7 fxyy, 8 fxxyy
+    const int val[3] = { 0, 1, 3 }, dy[3] = { 2, 4, 6 }, dyy[3] = { 5, 7, 8 };
+    for(int p = 0; p < 3; p++)
+        for(int a = 0; a < 2; a++) {
+            const double* lo = low + a * static_cast<size_t>(nt) * NODE_STRIDE;
+            const double* up = lo + NODE_STRIDE;
+            const double o = p == 0 ? off : 0;
+            const double fl = lo[val[p]] - o, fh = up[val[p]] - o;
+            const double f1l = lo[dy[p]], f1h = up[dy[p]], f2l = lo[dyy[p]], f2h = up[dyy[p]];
+            double* s = segments + k * CELL_COEFS + (2 * p + a) * 6;
+            s[0] = p == 0 && a == 0 ? off : fl;
+            s[1] = f1l;
+            s[2] = f2l;
+            s[3] = fma(-(0.5 * h), f1h + f1l, fh - fl);
+            s[4] = fma(-(0.5 * h), f2h + f2l, f1h - f1l);
+            s[5] = f2h - f2l;
+        }
+}
 }  // namespace
 
 void setError(const std::string& msg) { g_error = msg; }
@@ -247,12 +279,16 @@ DevicePotential* createDevicePotential(const std::vector<double>& radii,
                 P->cells.alloc(count * CELL_COEFS);
                 cellCoefsKernel<<<(count + 127) / 128, 128>>>(H.numSlots, V.nr, V.nt, V.gridR.cell, V.gridTau.cell,
                     V.spl2d, P->cells.ptr);
+                P->segments.alloc(count * CELL_COEFS);
+                cellSegmentsKernel<<<(count + 127) / 128, 128>>>(H.numSlots, V.nr, V.nt, V.gridTau.cell, V.spl2d,
+                    P->segments.ptr);
                 AGB_CUDA(cudaGetLastError());
                 AGB_CUDA(cudaStreamSynchronize(nullptr));
             }
         } else
             V.gridR = V.gridTau = GridView{};
         V.cells = P->cells.ptr;
+        V.segments = P->segments.ptr;
     } catch(...) {
         delete P;
         throw;

@@ -48,7 +48,7 @@ struct DevicePotential {
     MultipoleHost host;
     DevBuf<double> lnr, tau, lnrInvH, tauInvH, spl2d, spl1d, innerS, innerU, innerW, outerS, outerU, outerW;
     DevBuf<GridNode> gridCellR, gridCellTau;
-    DevBuf<double> cells, legendreNorm;
+    DevBuf<double> cells, segments, legendreNorm;
     DevBuf<unsigned short> gridLutR, gridLutTau;
     DevBuf<float> spl2d32;
     MultipoleView view;
