@@ -153,19 +153,21 @@ void runActions(const MultipoleView& M, const FudgeTables& F, long n, const doub
     const GLRules& gl = glRulesForCurrentDevice();
     const long pass = std::min(n, POINTS_PER_PASS);
     const bool predict = bp && bp->net;
-    // records, two work counters, the actions of a pass when the caller wants none, and the
-    // predictor's inputs and outputs
+    // records, two work counters, the actions of a pass when the caller wants none, the
+    // predictor's inputs and outputs, and the branch integrals of the angles
     const size_t recBytes = pass * (sizeof(FudgeRecord) + sizeof(FudgeEnds)) + 256;
     const size_t actBytes = act ? 0 : pass * 3 * sizeof(double);
-    const size_t featBytes = (predict ? pass * 9 * sizeof(float) : 0) + 256;
-    Scratch scratch(recBytes + actBytes + featBytes, stream);
+    const size_t featBytes = ((predict ? pass * 9 * sizeof(float) : 0) + 511) / 256 * 256;
+    const bool angles = ang || freq;
+    const size_t angleBytes = angles ? angleScratchBytes(pass) : 0;
+    Scratch scratch(recBytes + actBytes + featBytes + angleBytes, stream);
     FudgeRecord* rec = static_cast<FudgeRecord*>(scratch.ptr);
     FudgeEnds* ends = reinterpret_cast<FudgeEnds*>(rec + pass);
     unsigned long long* counter = reinterpret_cast<unsigned long long*>(ends + pass);
     double* actTmp = reinterpret_cast<double*>(static_cast<char*>(scratch.ptr) + recBytes);
     float* feat = predict ? reinterpret_cast<float*>(static_cast<char*>(scratch.ptr) + recBytes + actBytes) : nullptr;
     float* pred = predict ? feat + pass * 6 : nullptr;
-    const bool angles = ang || freq;
+    void* branchScratch = static_cast<char*>(scratch.ptr) + recBytes + actBytes + featBytes;
     BracketWidths widths{ { 0, 0, 0 } };
     if(predict) for(int k = 0; k < 3; k++) widths.w[k] = bp->widths[k];
     for(long first = 0; first < n; first += pass) {
@@ -198,7 +200,7 @@ void runActions(const MultipoleView& M, const FudgeTables& F, long n, const doub
             launchBracketTargets(count, rec, samples->target + 3 * first, samples->mask + 3 * first, stream);
         else if(angles)
             launchFudgeAngles(M, gl, count, rec, a, ang ? ang + 3 * first : nullptr,
-                freq ? freq + 3 * first : nullptr, stream);
+                freq ? freq + 3 * first : nullptr, branchScratch, counter + 1, stream);
         else
             launchFudgeIntegrals(M, gl, count, rec, a, counter + 1, g_actionMixed != 0, stream);
         mark(4);

@@ -8,6 +8,7 @@
 // actions alone are smooth in the limits and take the cells (fudge.cuh).
 #pragma once
 #include "fudge.cuh"
+#include "multipole_force.cuh"
 
 namespace agb {
 
@@ -248,72 +249,79 @@ static __device__ double scaleCubInverse(double ul, double ur, double u)
     return u < half ? s : 1 - s;
 }
 
-/// the three integrands of AxisymIntegrand::value with p in the denominator (n = -1), from one
-/// F(tau): (tau-Delta^2)^-1 [E], (tau-Delta^2)^-1 tau^-1 [I3], (tau-Delta^2)^-2 with the singular
-/// part at nu_max removed [Lz] (src/actions_staeckel.cpp:276-299)
-struct InverseMomentumTerms { double e, i3, lz; };
+/// the integrals over one branch of a point that its angles and frequencies need: those of the inverse
+/// momentum and (over the full range) of the momentum
+struct BranchSums { double e, i3, lz, act; };
 
-static __device__ InverseMomentumTerms inverseMomentumTerms(double ft, double tau, double D2, double nuMax,
-    double dfdnuMax)
-{
-    InverseMomentumTerms t{ 0, 0, 0 };
-    const double tmd = tau - D2;
-    const double p2 = ft / (2 * pow2(tmd) * tau);
-    if(p2 < 0) return t;
-    const double r = 1 / sqrt(p2);
-    double v = r / tmd;
-    t.e = isFinite(v) ? v : 0;
-    v = r / tmd / tau;
-    t.i3 = isFinite(v) ? v : 0;
-    v = r / pow2(tmd);
-    if(tmd < 0) v += sqrt(2 * nuMax / dfdnuMax / (tau - nuMax)) / tmd;
-    t.lz = isFinite(v) ? v : 0;
-    return t;
-}
+/// the branch integrals of a point, in the order of the tasks of angleIntegralKernel
+enum { BRANCH_LAMBDA = 0, BRANCH_NU = 1, BRANCH_LAMBDA_PART = 2, BRANCH_NU_PART = 3, NUM_BRANCHES = 4 };
 
-/// GL rule of the requested order (the next tabulated one at or above it)
-static __device__ __forceinline__ int glRule(const GLRules& gl, int order, const double** x, const double** w)
-{
-    int N = order < 1 ? 1 : order;
-    while(gl.offset[N] < 0) N++;
-    *x = gl.nodes + gl.offset[N];
-    *w = gl.weights + gl.offset[N];
-    return N;
-}
+/// what the branch integrals of a point share: dF/dtau at nu_max and the scaled positions of the point
+/// within its ranges (the upper ends of the partial integrals)
+struct AngleSetup { double dfdnuMax, yl, yn; };
 
-/** the inverse-momentum integrals of one branch over the scaled interval [0, y] of [lo, hi]
-    (integrateGL(ScaledIntegrand<ScalingCub>, 0, y, N), src/math_core.cpp:1191-1205); with
-    ACT also the action integral (p in the numerator) over the same nodes, when y = 1 */
-template<bool ACT>
-static __device__ InverseMomentumTerms branchIntegrals(const FudgeFunction& fnc, const GLRules& gl, int order,
-    double lo, double hi, double y, double nuMax, double dfdnuMax, double* act)
+static __device__ AngleSetup fudgeAngleSetup(const MultipoleView& M, const FudgeRecord& rec, bool parts)
 {
-    InverseMomentumTerms sum{ 0, 0, 0 };
-    if(ACT) *act = 0;
-    if(y == 0) return sum;
-    const double *x, *w;
-    const int N = glRule(gl, order, &x, &w);
-    double sa = 0;
-    for(int i = 0; i < N; i++) {
-        const double xi = ldg(x + i), wi = ldg(w + i);
-        double duds;
-        const double tau = unscaleCub(lo, hi, y * xi + 0 * (1 - xi), &duds);
-        const double ft = fnc.value(tau);
-        const InverseMomentumTerms t = inverseMomentumTerms(ft, tau, fnc.D2, nuMax, dfdnuMax);
-        sum.e += wi * (t.e * duds);
-        sum.i3 += wi * (t.i3 * duds);
-        sum.lz += wi * (t.lz * duds);
-        if(ACT) {
-            const double tmd = tau - fnc.D2;
-            const double p2 = ft / (2 * pow2(tmd) * tau);
-            double v = p2 < 0 ? 0 : sqrt(p2);
-            if(!isFinite(v)) v = 0;
-            sa += wi * (v * duds);
-        }
+    FudgeFunction fnc;
+    loadFudgeFunction(M, rec, fnc);
+    const FudgeLimits lim = fudgeLimitsFinish(rec);
+    AngleSetup a{ 0, 0, 0 };
+    double unused;
+    fnc.eval<true, false>(lim.nu_max, &unused, &a.dfdnuMax, nullptr);
+    if(parts) {
+        a.yl = scaleCubInverse(lim.lambda_min, lim.lambda_max, rec.lambda);
+        a.yn = lim.nu_max == 0 ? 0 : scaleCubInverse(0, lim.nu_max, fabs(rec.nu));
     }
-    sum.e *= y; sum.i3 *= y; sum.lz *= y;
-    if(ACT) *act = sa * y;
-    return sum;
+    return a;
+}
+
+/// F(tau) of one branch (FudgeFunction::eval, to the bit) in a potential with cells, without calls;
+/// D2inv = 1 / D2
+static __device__ __forceinline__ double branchValue(const FudgeFunction& f, double D2inv, double tau)
+{
+    const MultipoleView& M = *f.M;
+    const bool lambda = tau >= f.D2;
+    const double lam = lambda ? tau : f.lambda, n = lambda ? fabs(f.nu) : tau;
+    const double mult = lambda ? lam - n : n - lam, I = lambda ? f.Ilam : f.Inu;
+    const double absnu = fabs(n), lmd = lam - f.D2, nmd = absnu - f.D2;
+    if(nmd > 0 || lmd < 0) return NAN;
+    // coordinates that leave the range of normal numbers take the library's roots
+    const double R2 = lmd * (1 - quotient(absnu, f.D2, D2inv)), z2 = quotient(lam * absnu, f.D2, D2inv);
+    const bool usual = R2 > 1e-200 && R2 < 1e200 && z2 > 1e-200 && z2 < 1e200;
+    const double R = usual ? squareRoot(R2) : sqrt(R2), z = (usual ? squareRoot(z2) : sqrt(z2)) * (n >= 0 ? 1 : -1);
+    const double rsq = sumProducts(z, z, R, R);
+    const double Phi = inCells(M, rsq) ? valueInterp2d(M, R, z) : valuePowerLaw(rsq < M.rInnerSq ? M.inner : M.outer, R, z);
+    const double tmd = tau - f.D2;
+    return fma(-f.L2h, tau, tmd != 0 ? fma(-Phi, mult, fma(f.E, tau, -I)) * tmd : 0);
+}
+
+/// one node (abscissa x, weight w) of a branch integral over the scaled interval [0, y] of [lo, hi]
+/// (integrateGL(ScaledIntegrand<ScalingCub>, 0, y, N), src/math_core.cpp:1191-1205) added to its sums: the three
+/// integrands of AxisymIntegrand::value with p in the denominator (n = -1), from one F(tau):
+/// (tau-Delta^2)^-1 [E], (tau-Delta^2)^-1 tau^-1 [I3], (tau-Delta^2)^-2 with the singular part at nu_max
+/// removed [Lz] (src/actions_staeckel.cpp:276-299), and p itself.  The quotients are rounded from shared
+/// reciprocals; where one of them has no finite value its term is left out in either case.
+/// CELLS: the potential has cells (2-D splines).
+template<bool CELLS>
+static __device__ __forceinline__ void addBranchNode(const FudgeFunction& fnc, double D2inv, double x, double w,
+    double lo, double hi, double y, double nuMax, double dfdnuMax, BranchSums& sum)
+{
+    const double s = y * x;
+    const double duds = (hi - lo) * 6 * s * (1 - s);
+    const double tau = sumProducts(hi * pow2(s), 3 - 2 * s, lo * pow2(1 - s), 1 + 2 * s);
+    const double ft = CELLS ? branchValue(fnc, D2inv, tau) : fnc.value(tau);
+    const double tmd = tau - fnc.D2, tmd2 = pow2(tmd), den = 2 * tmd2 * tau;
+    const double p2 = quotient(ft, den, reciprocal(den));
+    if(p2 < 0) return;
+    const double root = squareRoot(p2), r = reciprocal(root), tmdInv = reciprocal(tmd);
+    double v = quotient(r, tmd, tmdInv);
+    if(isFinite(v)) sum.e = fma(w, v * duds, sum.e);
+    v = quotient(v, tau, reciprocal(tau));
+    if(isFinite(v)) sum.i3 = fma(w, v * duds, sum.i3);
+    v = quotient(r, tmd2, reciprocal(tmd2));
+    if(tmd < 0) v += sqrt(2 * nuMax / dfdnuMax / (tau - nuMax)) / tmd;
+    if(isFinite(v)) sum.lz = fma(w, v * duds, sum.lz);
+    if(isFinite(root)) sum.act = fma(w, root * duds, sum.act);
 }
 
 /// 2 pi wrap of an angle into [0, 2 pi) (math::wrapAngle, src/math_core.cpp:149-157; NaN -> 0)
@@ -326,27 +334,21 @@ static __device__ __forceinline__ double wrapAngle(double x)
 /** Actions, frequencies and angles of a prepared point whose roots are found (evalAxisym,
     src/actions_staeckel.cpp:645-670): computeActions (:604-619), computeActionDerivatives
     (:489-527), computeIntDerivatives (:532-560), computeGenFuncDerivatives (:566-600) and
-    computeAngles (:624-636).  The action integrals and the derivative integrals share their
-    potential evaluations (same nodes); ang / freq may be null. */
-static __device__ void fudgeAnglesFrequencies(const MultipoleView& M, const GLRules& gl, const FudgeRecord& rec,
-    double* act, double* ang, double* freq)
+    computeAngles (:624-636), from the sums of its branch integrals (scaled by the upper ends of their
+    intervals).  ang / freq may be null. */
+static __device__ void fudgeAnglesFrequencies(const MultipoleView& M, const FudgeRecord& rec, const AngleSetup& setup,
+    const BranchSums* sums, double* act, double* ang, double* freq)
 {
-    FudgeFunction fnc;
-    loadFudgeFunction(M, rec, fnc);
     const FudgeLimits lim = fudgeLimitsFinish(rec);
-    const double D2 = rec.D2, Lz = rec.Lz;
-    double dfdnuMax, unused;
-    fnc.eval<true, false>(lim.nu_max, &unused, &dfdnuMax, nullptr);
-    // action derivatives over (E, I3, Lz), full ranges; the actions from the same nodes
-    double Jr, Jz;
-    InverseMomentumTerms L = branchIntegrals<true>(fnc, gl, lim.order, lim.lambda_min, lim.lambda_max, 1,
-        lim.nu_max, dfdnuMax, &Jr);
-    const InverseMomentumTerms N = branchIntegrals<true>(fnc, gl, lim.order, 0, lim.nu_max, 1,
-        lim.nu_max, dfdnuMax, &Jz);
-    act[0] = Jr / M_PI;
-    act[1] = Jz / M_PI * 2;
+    const double D2 = rec.D2, Lz = rec.Lz, dfdnuMax = setup.dfdnuMax;
+    BranchSums L = sums[BRANCH_LAMBDA];
+    const BranchSums N = sums[BRANCH_NU];
+    act[0] = L.act / M_PI;
+    act[1] = N.act / M_PI * 2;
     if(lim.lambda_min == lim.lambda_max) {      // limitingIntegralValue, :307-323
         const double tau = lim.lambda_min, tmd = tau - D2;
+        FudgeFunction fnc;
+        loadFudgeFunction(M, rec, fnc);
         double d2, v0;
         fnc.eval<false, true>(tau, &v0, nullptr, &d2);
         const double base = 2 * M_PI * sqrt(-tau / d2) * fabs(tmd);
@@ -362,7 +364,7 @@ static __device__ void fudgeAnglesFrequencies(const MultipoleView& M, const GLRu
     const double dJzdLz = -Lz * (N.lz + singpart) / (2 * M_PI);
     // inverse matrix: frequencies and the derivatives of I3 over the actions
     double Or, Oz, Ophi, dI3dJr, dI3dJz, dI3dJphi;
-    const double det = dJrdE * dJzdI3 - dJrdI3 * dJzdE;
+    const double det = sumProducts(dJrdE, dJzdI3, -dJrdI3, dJzdE);
     if(lim.nu_max == 0 || det == 0) {
         Or = 1 / dJrdE;
         Ophi = -dJrdLz / dJrdE;
@@ -370,31 +372,26 @@ static __device__ void fudgeAnglesFrequencies(const MultipoleView& M, const GLRu
     } else {
         Or = dJzdI3 / det;
         Oz = -dJrdI3 / det;
-        Ophi = (dJrdI3 * dJzdLz - dJrdLz * dJzdI3) / det;
+        Ophi = sumProducts(dJrdI3, dJzdLz, -dJrdLz, dJzdI3) / det;
         dI3dJr = -dJzdE / det;
         dI3dJz = dJrdE / det;
-        dI3dJphi = -(dJrdE * dJzdLz - dJrdLz * dJzdE) / det;
+        dI3dJphi = -sumProducts(dJrdE, dJzdLz, -dJrdLz, dJzdE) / det;
     }
     if(freq) { freq[0] = Or; freq[1] = Oz; freq[2] = Ophi; }
     if(!ang) return;
     // derivatives of the generating function over (E, I3, Lz): integrals up to the point
     const double signl = rec.valid & REC_LDOT_POS ? 1 : -1, signn = rec.valid & REC_NDOT_NU_POS ? 1 : -1;
     const double absnu = fabs(rec.nu);
-    const double yl = scaleCubInverse(lim.lambda_min, lim.lambda_max, rec.lambda);
-    const double yn = lim.nu_max == 0 ? 0 : scaleCubInverse(0, lim.nu_max, absnu);
-    const InverseMomentumTerms Lp = branchIntegrals<false>(fnc, gl, lim.order, lim.lambda_min, lim.lambda_max, yl,
-        lim.nu_max, dfdnuMax, nullptr);
-    const InverseMomentumTerms Np = branchIntegrals<false>(fnc, gl, lim.order, 0, lim.nu_max, yn,
-        lim.nu_max, dfdnuMax, nullptr);
+    const BranchSums Lp = sums[BRANCH_LAMBDA_PART], Np = sums[BRANCH_NU_PART];
     const double dSdE = signl * Lp.e / 4 + signn * Np.e / 4;
     const double dSdI3 = signl * -Lp.i3 / 4 + signn * -Np.i3 / 4;
     const double singS = 2 * sqrt(-2 * lim.nu_max / dfdnuMax / dmn) *
         (atan(sqrt(lim.nu_max / dmn)) - atan(sqrt((lim.nu_max - absnu) / dmn)));
     const double dSdLz = Lz == 0 ? 0 : rec.phi + signl * -Lz * Lp.lz / 4 + signn * -Lz * (Np.lz + singS) / 4;
     const bool addPi = (rec.valid & REC_NUDOT_NEG) && Lz != 0;
-    ang[0] = wrapAngle(dSdE * Or + dSdI3 * dI3dJr + dSdLz * 0);
-    ang[1] = wrapAngle(dSdE * Oz + dSdI3 * dI3dJz + dSdLz * 0 + M_PI * addPi);
-    ang[2] = wrapAngle(dSdE * Ophi + dSdI3 * dI3dJphi + dSdLz * 1);
+    ang[0] = wrapAngle(sumProducts(dSdE, Or, dSdI3, dI3dJr) + dSdLz * 0);
+    ang[1] = wrapAngle(sumProducts(dSdE, Oz, dSdI3, dI3dJz) + dSdLz * 0 + M_PI * addPi);
+    ang[2] = wrapAngle(sumProducts(dSdE, Ophi, dSdI3, dI3dJphi) + dSdLz * 1);
 }
 
 }  // namespace agb

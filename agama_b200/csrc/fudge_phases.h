@@ -42,8 +42,9 @@ void launchFudgeIntegrals(const MultipoleView& M, const GLRules& gl, long n, con
 
 /// phase 3 with angles / frequencies: actions into act (n x 3, Jphi already there), frequencies
 /// (Omega_r, Omega_z, Omega_phi) and angles (theta_r, theta_z, theta_phi) into freq / ang when
-/// not null; one point per thread
+/// not null; scratch: angleScratchBytes(n) for the branch integrals, counter: 8 bytes, zeroed here
+size_t angleScratchBytes(long n);
 void launchFudgeAngles(const MultipoleView& M, const GLRules& gl, long n, const FudgeRecord* rec, double* act,
-    double* ang, double* freq, cudaStream_t stream);
+    double* ang, double* freq, void* scratch, unsigned long long* counter, cudaStream_t stream);
 
 }  // namespace agb

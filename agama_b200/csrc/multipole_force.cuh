@@ -66,38 +66,61 @@ struct SegmentBasis {
     }
 };
 
-/** spline2dCell for value and gradient away from the upper nodes of a cell, from its segments in the
-    second direction (MultipoleView::segments): what depends on the table alone -- the three defects of
-    each segment, a quarter of the arithmetic -- is tabulated, by the same operations.
-    (y: the basis in tau, x: in ln r, hx: the width of the cell in ln r) */
-__device__ __forceinline__ void segmentCell(const double* __restrict__ c, const SegmentBasis& x, double hx,
-    const SegmentBasis& y, double* z, double* zx, double* zy)
+/** The values (and with SLOPE the tau derivatives) of the six functions of a cell at a tau within it
+    (MultipoleView::segments): what depends on the table alone -- the three defects of each segment, a
+    quarter of the arithmetic of spline2dCell -- is tabulated, by the same operations.  At the cell's upper
+    tau node (the last one of the grid, on the axis) they are the node values, without round-off; node:
+    the spline node (xlow, yupp), row: the distance to (xupp, yupp).  F[0] and F[1] are relative to off.
+    (The upper ln r node is never met: the last one lies beyond the switch to the outer expansion.) */
+template<bool SLOPE>
+__device__ __forceinline__ void cellSegments(const double* __restrict__ c, const double* node, size_t row, bool upper,
+    const SegmentBasis& y, double* F, double* G, double* off)
 {
-    double F[6], G[6], off = 0;
+    if(upper) {
+        const int val[3] = { 0, 1, 3 }, dy[3] = { 2, 4, 6 };
+        *off = ldg(node);
+#pragma unroll
+        for(int p = 0; p < 3; p++) {
+            F[2 * p] = p == 0 ? 0 : ldg(node + val[p]);
+            F[2 * p + 1] = p == 0 ? ldg(node + row) - *off : ldg(node + row + val[p]);
+            if(SLOPE) { G[2 * p] = ldg(node + dy[p]); G[2 * p + 1] = ldg(node + row + dy[p]); }
+        }
+        return;
+    }
 #pragma unroll
     for(int p = 0; p < 6; p += 2) {
         double w[12];
         ldg4(c + 6 * p, w);
         ldg4(c + 6 * p + 4, w + 4);
         ldg4(c + 6 * p + 8, w + 8);
-        if(p == 0) { off = w[0]; w[0] = 0; }
+        if(p == 0) { *off = w[0]; w[0] = 0; }
 #pragma unroll
         for(int a = 0; a < 2; a++) {
             const double* s = w + 6 * a;
             F[p + a] = y.value(s[0], s[1], s[2], s[3], s[4], s[5]);
-            G[p + a] = y.slope(s[1], s[2], s[3], s[4], s[5]);
+            if(SLOPE) G[p + a] = y.slope(s[1], s[2], s[3], s[4], s[5]);
         }
     }
-    auto defects = [&](const double* f, double* d) {
-        d[0] = fma(-(0.5 * hx), f[3] + f[2], f[1] - f[0]);
-        d[1] = fma(-(0.5 * hx), f[5] + f[4], f[3] - f[2]);
-        d[2] = f[5] - f[4];
-    };
-    double d[3];
-    defects(F, d);
+}
+
+/// the defects of the segment in ln r from its six values (quinticSegmentR), hx: its width
+__device__ __forceinline__ void segmentDefects(const double* f, double hx, double* d)
+{
+    d[0] = fma(-(0.5 * hx), f[3] + f[2], f[1] - f[0]);
+    d[1] = fma(-(0.5 * hx), f[5] + f[4], f[3] - f[2]);
+    d[2] = f[5] - f[4];
+}
+
+/// spline2dCell for value and gradient from the cell's segments
+__device__ __forceinline__ void segmentCell(const double* __restrict__ c, const double* node, size_t row, bool upper,
+    const SegmentBasis& x, double hx, const SegmentBasis& y, double* z, double* zx, double* zy)
+{
+    double F[6], G[6], off, d[3];
+    cellSegments<true>(c, node, row, upper, y, F, G, &off);
+    segmentDefects(F, hx, d);
     *z = x.value(F[0], F[2], F[4], d[0], d[1], d[2]) + off;
     *zx = x.slope(F[2], F[4], d[0], d[1], d[2]);
-    defects(G, d);
+    segmentDefects(G, hx, d);
     *zy = x.value(G[0], G[2], G[4], d[0], d[1], d[2]);
 }
 
@@ -107,21 +130,8 @@ __device__ __forceinline__ void segmentCell(const double* __restrict__ c, const 
     falls), so nothing is kept per harmonic.
     G > 1: the lanes of a group take G harmonics at a time, one each, and every lane adds all of them
     in the same order from the lane that evaluated it, so every G gives the same bits.
-    MIXED: the m != 0 harmonics from the FP32 table.
-    NODES: the cells from the node values, for points at an upper node of either direction (the last
-    ones of the grids, where the node values are taken without round-off). */
-template<int KIND, int G, bool MIXED, bool NODES>
-__device__ __forceinline__ void forceInterp2d(const MultipoleView& M, double R, double z, double phi, double* pot,
-    CylDerivs* g);
-
+    MIXED: the m != 0 harmonics from the FP32 table. */
 template<int KIND, int G, bool MIXED>
-__device__ __noinline__ void forceAtUpperNode(const MultipoleView& M, double R, double z, double phi, double* pot,
-    CylDerivs* g)
-{
-    forceInterp2d<KIND, G, MIXED, true>(M, R, z, phi, pot, g);
-}
-
-template<int KIND, int G, bool MIXED, bool NODES>
 __device__ __forceinline__ void forceInterp2d(const MultipoleView& M, double R, double z, double phi, double* pot,
     CylDerivs* g)
 {
@@ -132,25 +142,21 @@ __device__ __forceinline__ void forceInterp2d(const MultipoleView& M, double R, 
     const bool inside = logr >= M.gridR.x0 && logr <= M.gridR.xEnd && tau >= M.gridTau.x0 && tau <= M.gridTau.xEnd;
     double xl, xh, yl, yh, xhi, yhi;
     const int xs = gridCell(M.gridR, logr, &xl, &xh, &xhi), ys = gridCell(M.gridTau, tau, &yl, &yh, &yhi);
-    if(!NODES && (logr == xh || tau == yh)) {
-        forceAtUpperNode<KIND, G, MIXED>(M, R, z, phi, pot, g);
-        return;
-    }
+    const bool upper = tau == yh;
     const SegmentBasis bx(logr, xl, xh, xhi), by(tau, yl, yh, yhi);
     const size_t slotStride = static_cast<size_t>(M.nr) * M.nt * NODE_STRIDE;
     const size_t segmentStride = static_cast<size_t>(M.nr - 1) * (M.nt - 1) * CELL_COEFS;
     const double* segments = M.segments + (static_cast<size_t>(xs) * (M.nt - 1) + ys) * CELL_COEFS;
+    const double* nodes = M.spl2d + (static_cast<size_t>(xs) * M.nt + ys + 1) * NODE_STRIDE;
     auto cell = [&](int s, double* P, double* Dr, double* Dt) {
         const int slot = M.fastSlot[s];
-        double rr, rt, tt;
-        if(MIXED && s > 0)      // m != 0 (angular) harmonics in FP32, the radial m = 0 one in FP64
+        if(MIXED && s > 0) {    // m != 0 (angular) harmonics in FP32, the radial m = 0 one in FP64
+            double rr, rt, tt;
             spline2dCell32<3>(M.spl2d32 + slot * slotStride, M.nt, xs, ys, logr, xl, xh, tau, yl, yh,
                 P, Dr, Dt, &rr, &rt, &tt);
-        else if(NODES)
-            spline2dCell<3>(M.spl2d + slot * slotStride, M.nt, xs, ys, logr, xl, xh, tau, yl, yh, xhi, yhi,
-                P, Dr, Dt, &rr, &rt, &tt);
-        else
-            segmentCell(segments + slot * segmentStride, bx, xh - xl, by, P, Dr, Dt);
+        } else
+            segmentCell(segments + slot * segmentStride, nodes + slot * slotStride, static_cast<size_t>(M.nt) * NODE_STRIDE,
+                upper, bx, xh - xl, by, P, Dr, Dt);
         if(!inside) *P = *Dr = *Dt = NAN;
     };
     const int numHarm = KIND == EVAL_AXI ? 1 : M.nFast;
@@ -341,6 +347,59 @@ __device__ __forceinline__ void powerLawTerms(const PowerLawView& A, double R, d
     g->dphi = gp;
 }
 
+/// the potential alone of an axisymmetric expansion at (R, z) inside its 2-D splines, to the bit that of
+/// evalInterp2dFast
+__device__ __forceinline__ double valueInterp2d(const MultipoleView& M, double R, double z)
+{
+    const double r = squareRoot(sumProducts(z, z, R, R)), logr = log(r), rpRinv = reciprocal(r + fabs(R));
+    const double tau = R == 0 ? signOf(z) : z * rpRinv;
+    const bool inside = logr >= M.gridR.x0 && logr <= M.gridR.xEnd && tau >= M.gridTau.x0 && tau <= M.gridTau.xEnd;
+    double xl, xh, yl, yh, xhi, yhi, F[6], off, d[3];
+    const int xs = gridCell(M.gridR, logr, &xl, &xh, &xhi), ys = gridCell(M.gridTau, tau, &yl, &yh, &yhi);
+    const SegmentBasis x(logr, xl, xh, xhi), y(tau, yl, yh, yhi);
+    const size_t slot = M.fastSlot[0];
+    cellSegments<false>(M.segments + ((slot * (M.nr - 1) + xs) * (M.nt - 1) + ys) * CELL_COEFS,
+        M.spl2d + ((slot * M.nr + xs) * M.nt + ys + 1) * NODE_STRIDE, static_cast<size_t>(M.nt) * NODE_STRIDE, tau == yh, y,
+        F, nullptr, &off);
+    segmentDefects(F, xh - xl, d);
+    double P = x.value(F[0], F[2], F[4], d[0], d[1], d[2]) + off;
+    if(!inside) P = NAN;
+    if(M.logScaling) P = reciprocal(M.invPhi0 - exp(P));
+    return P;
+}
+
+/// the potential alone of an axisymmetric asymptotic expansion (evalPowerLaw): one short loop, inline
+__device__ __forceinline__ double valuePowerLaw(const PowerLawView& A, double R, double z)
+{
+    const HarmIndices& ind = A.ind;
+    const double rsq = sumProducts(z, z, R, R), dlogr = log(rsq / A.r0sq) * 0.5;
+    const int lmax = (A.inner && rsq < A.r0sq * 1e-16) || (!A.inner && rsq > A.r0sq * 1e16) ? 0 : ind.lmax;
+    const double tau = z == 0 ? 0 : z / (sqrt(rsq) + R);
+    const double ct = 2 * tau / (1 + tau * tau);
+    double prefact = PMM_NORM_DEV[0], sum = 0, Plm1 = 1, Plm = 1, Plm2 = 0;
+    for(int l = 0; l <= lmax; l++) {
+        if(l == 1) Plm = ct * Plm1;
+        else if(l > 1) {
+            const double num = sumProducts(ct * (2 * l - 1), Plm1, -(l - 1), Plm2), d = l;
+            Plm = quotient(num, d, 1 / d);
+        }
+        if(l > 0) prefact *= ldg(A.norm + l);
+        if(l % ind.step == 0) {
+            const int c = HarmIndices::index(l, 0);
+            const double s = ldg(A.S + c), u = ldg(A.U + c), w = ldg(A.W + c), v = A.inner ? l : -l - 1;
+            const double rv = v != 0 ? exp(dlogr * v) : 1;
+            const double rs = s != v ? (s != 0 && u != 0 ? exp(dlogr * s) : 1) : rv;
+            const double urs = u * rs * (s != v || u == 0 ? 1 : dlogr);
+            const double C = __dadd_rn(urs, w * rv) + (v == 0 ? A.Q * rsq / A.r0sq : 0);
+            if(lmax == 0) return C;
+            sum = fma(Plm * prefact * C, 2 * SQRT_PI, sum);
+        }
+        Plm2 = Plm1;
+        Plm1 = Plm;
+    }
+    return sum;
+}
+
 /// beyond the 2-D splines: asymptotic expansions (and 1-D splines); out of line
 static __device__ __noinline__ void forceBeyond(const MultipoleView& M, double R, double z, double phi, double* pot, CylDerivs* g)
 {
@@ -390,7 +449,7 @@ __device__ __forceinline__ void evalForceCar(const MultipoleView& M, double x, d
         CylHess h;
         evalMultipoleCyl<3, KIND>(M, R, z, phi, pot, &g, &h);
     } else if(inCells(M, rsq))
-        forceInterp2d<KIND, G, MIXED, false>(M, R, z, phi, pot, &g);
+        forceInterp2d<KIND, G, MIXED>(M, R, z, phi, pot, &g);
     else
         forceBeyond(M, R, z, phi, pot, &g);
     grad[0] = noAzimuth ? g.dR * dRdx : sumProducts(g.dR, dRdx, g.dphi, dphidx);
