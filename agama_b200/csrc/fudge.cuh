@@ -96,6 +96,40 @@ static __device__ __forceinline__ double deltaLookup(const FudgeTables& F, doubl
     return T * (U * zll + u * zlu) + t * (U * zul + u * zuu);
 }
 
+/** An axisymmetric asymptotic expansion (evalPowerLaw) at (R, z): the potential, and with DER its derivatives
+    over ln r and over the latitude.  One loop over l with the Legendre recurrence, inline. */
+template<bool DER>
+__device__ __forceinline__ void powerLawAxi(const PowerLawView& A, double rsq, double R, double z, double* Phi, double* px,
+    double* ppsi)
+{
+    const double dlogr = 0.5 * log(rsq / A.r0sq);
+    const int lmax = (A.inner && rsq < A.r0sq * 1e-16) || (!A.inner && rsq > A.r0sq * 1e16) ? 0 : A.ind.lmax;
+    const double rinv = rsq > 0 ? 1 / sqrt(rsq) : 0, ct = z * rinv, st = R * rinv;
+    double sum = 0, sumr = 0, sumt = 0, P = 1, Pm1 = 0, dP = 0, dPm1 = 0;  // Legendre P_l and dP_l / d(ct)
+    for(int l = 0; l <= lmax; l++) {
+        if(l > 0) {
+            const double p = ((2 * l - 1) * ct * P - (l - 1) * Pm1) / l;
+            const double d = DER ? dPm1 + (2 * l - 1) * P : 0;
+            Pm1 = P; P = p;
+            dPm1 = dP; dP = d;
+        }
+        if(l % A.ind.step) continue;
+        const int c = HarmIndices::index(l, 0);
+        const double s = ldg(A.S + c), u = ldg(A.U + c), w = ldg(A.W + c), v = A.inner ? l : -l - 1;
+        const double rv = v != 0 ? exp(dlogr * v) : 1;
+        const double rs = s != v ? (s != 0 && u != 0 ? exp(dlogr * s) : 1) : rv;
+        const double urs = u * rs * (s != v || u == 0 ? 1 : dlogr), wrv = w * rv;
+        const double qr2 = v == 0 ? A.Q * rsq / A.r0sq : 0, norm = lmax == 0 ? 1 : sqrt(2 * l + 1.);
+        sum += (urs + wrv + qr2) * (norm * P);
+        if(DER) {
+            sumr += (urs * s + wrv * v + (s != v ? 0 : u * rs) + 2 * qr2) * (norm * P);
+            sumt += (urs + wrv + qr2) * (norm * dP);
+        }
+    }
+    *Phi = sum;
+    if(DER) { *px = sumr; *ppsi = sumt * st; }      // d(ct) / dpsi = cos(psi) = sin(theta)
+}
+
 /** The fudge's auxiliary function F(tau) along one of the two coordinates of a point (the other one
     stays at its value there); AxisymFunctionFudge::evalDeriv, src/actions_staeckel.cpp:202-252, with
     prolate spheroidal -> cylindrical coordinates from src/coord.cpp:266-291.
@@ -132,8 +166,10 @@ struct FudgeBranch {
         c2 = sqrt((lam ? n : lambda) * inv);
     }
 
-    /// F(tau), and with DER its derivative
-    template<bool DER>
+    /// F(tau), and with DER its derivative.  CELLS: the potential has cells (2-D splines), and beyond them
+    /// the asymptotic expansions are evaluated inline: with a call there the registers saved around it cost the
+    /// searches and integrals their hot path (370 B of spills)
+    template<bool DER, bool CELLS>
     __device__ __forceinline__ void eval(const MultipoleView& M, double tau, double* val, double* der) const
     {
         const double tmd = tau - D2;
@@ -158,11 +194,15 @@ struct FudgeBranch {
                 Phi = rcpNormal(M.invPhi0 - ex);
                 if(DER) { const double d = Phi * Phi * ex; px *= d; ppsi *= d; }
             }
-        } else {
-            CylDerivs g; CylHess h;
-            evalBeyondCells<DER ? 3 : 1>(M, R, z, 0, &Phi, &g, &h);
+        } else if(CELLS) {
             r2inv = 1 / rsq;
-            if(DER) { px = R * g.dR + z * g.dz; ppsi = R * g.dz - z * g.dR; }
+            powerLawAxi<DER>(rsq < M.rInnerSq ? M.inner : M.outer, rsq, R, z, &Phi, &px, &ppsi);
+        } else {
+            BeyondCells b;
+            evalBeyondCells<DER ? 3 : 1>(M, R, z, 0, &b);
+            Phi = b.pot;
+            r2inv = 1 / rsq;
+            if(DER) { px = R * b.g.dR + z * b.g.dz; ppsi = R * b.g.dz - z * b.g.dR; }
         }
         const double mult = tau - mo;
         *val = (E * tau - I - Phi * mult) * tmd - L2h * tau;
@@ -172,10 +212,11 @@ struct FudgeBranch {
             *der = E * (tau + tmd) - L2h - I - (mult + tmd) * Phi - (tmd != 0 ? tmd * mult * dPhi : 0);
         }
     }
+    template<bool CELLS>
     __device__ __forceinline__ double value(const MultipoleView& M, double tau) const
     {
         double v;
-        eval<false>(M, tau, &v, nullptr);
+        eval<false, CELLS>(M, tau, &v, nullptr);
         return v;
     }
 };
@@ -208,7 +249,7 @@ static __device__ __noinline__ void fudgeSecondAt(const MultipoleView& M, const 
 /// F(tau) out of line, for the rare single values of phase 1 and the angles
 static __device__ __noinline__ double fudgeValueAt(const MultipoleView& M, const FudgeBranch& f, double tau)
 {
-    return f.value(M, tau);
+    return f.value<false>(M, tau);
 }
 
 /// State of one point between the phases of the action computation: the point in prolate
@@ -242,6 +283,7 @@ struct FudgeEnds { double fPos, dfPos, fD2, dfD2, fNu, dfNu; };
     for nu_max and lambda_min; with semiInf (lambda_max) F(tau)/tau^2 on
     [u0, inf) mapped to s in [0, 1] by the semi-infinite scaling, AxisymScaledForRootfinder inside
     ScaledFnc<ScalingSemiInf>, src/actions_staeckel.cpp:329-354, src/math_core.h:214-232). */
+template<bool CELLS>
 __device__ __forceinline__ void limitRootEval(const MultipoleView& M, const FudgeBranch& f, bool semiInf, double u0,
     double x, double* v, double* d)
 {
@@ -253,7 +295,7 @@ __device__ __forceinline__ void limitRootEval(const MultipoleView& M, const Fudg
     }
     const bool far = semiInf && !(tau <= 1e100);
     double fval = 0, fder = 0;
-    if(!far) f.eval<true>(M, tau, &fval, &fder);
+    if(!far) f.eval<true, CELLS>(M, tau, &fval, &fder);
     if(!semiInf) { *v = fval; *d = fder; }
     else if(far) { *v = f.E; *d = NAN; }
     else {
@@ -269,42 +311,59 @@ __device__ __forceinline__ void loadFudgeBranch(const FudgeRecord& r, bool lambd
     f.set(lambdaBranch, r.lambda, r.nu, r.D2, r.E, r.Lz, r.I3, r.flambda, r.fnu);
 }
 
-/// out-of-line value of the potential in the equatorial plane or on the axis at squared radius rsq
-static __device__ __noinline__ double potentialOnAxes(const MultipoleView& M, double rsq, int axis)
+/// the potential of the cells in the equatorial plane or on the axis at squared radius rsq (inCells)
+__device__ __forceinline__ double cellsOnAxes(const MultipoleView& M, double rsq, int axis)
 {
-    double Phi;
-    if(inCells(M, rsq)) {
-        const double logr = 0.5 * log(rsq);
-        double xl, xh, xi, yl, yh, yi, dummy;
-        const int ix = gridCell(M.gridR, logr, &xl, &xh, &xi), iy = gridCell(M.gridTau, axis, &yl, &yh, &yi);
-        cellPolynomial<1>(M.cells + (static_cast<size_t>(ix) * (M.nt - 1) + iy) * CELL_COEFS, (logr - xl) * xi,
-            (axis - cellAnchor(yl, yh)) * yi, &Phi, &dummy, &dummy, &dummy, &dummy, &dummy);
-        if(M.logScaling) Phi = rcpNormal(M.invPhi0 - exp(Phi));
-    } else {
-        const double r = sqrt(rsq);
-        CylDerivs g; CylHess h;
-        evalBeyondCells<1>(M, axis ? 0 : r, axis ? r : 0, 0, &Phi, &g, &h);
-    }
-    return Phi;
+    const double logr = 0.5 * log(rsq);
+    double xl, xh, xi, yl, yh, yi, Phi, dummy;
+    const int ix = gridCell(M.gridR, logr, &xl, &xh, &xi), iy = gridCell(M.gridTau, axis, &yl, &yh, &yi);
+    cellPolynomial<1>(M.cells + (static_cast<size_t>(ix) * (M.nt - 1) + iy) * CELL_COEFS, (logr - xl) * xi,
+        (axis - cellAnchor(yl, yh)) * yi, &Phi, &dummy, &dummy, &dummy, &dummy, &dummy);
+    return M.logScaling ? rcpNormal(M.invPhi0 - exp(Phi)) : Phi;
+}
+
+/// the same at any radius
+__device__ __forceinline__ double potentialOnAxes(const MultipoleView& M, double rsq, int axis)
+{
+    if(inCells(M, rsq)) return cellsOnAxes(M, rsq, axis);
+    const double r = sqrt(rsq);
+    BeyondCells b;
+    evalBeyondCells<1>(M, axis ? 0 : r, axis ? r : 0, 0, &b);
+    return b.pot;
 }
 
 /** What phase 1 needs of the potential, from the cells: one evaluation with the Hessian at the point
     (R, |z|) gives F of both branches there up to F'', the value at (lambda, nu = 0) gives the
     integrals of motion and F(0), and the value on the axis F' at Delta^2.  (The node form evaluates
-    the potential six times.)  The same struct is the evaluator of fudgeLimitsSetup. */
+    the potential six times.)  The same struct is the evaluator of fudgeLimitsSetup.
+    FAST: for points inside the cells, without calls; `rare` is set where something else is needed. */
+template<bool FAST>
 struct CellPoint {
+    bool rare = false;
     double R, z, Phi, Phi0;
     CylDerivs g;
     CylHess h;
     const MultipoleView* view;
     const FudgeRecord* rec;
-    __device__ __noinline__ void locate(const MultipoleView& M, double R_, double z_)
+    __device__ __forceinline__ void locate(const MultipoleView& M, double R_, double z_)
     {
         view = &M;
         R = R_; z = fabs(z_);
-        evalCellsCyl<6, EVAL_AXI>(M, R, z, 0, &Phi, &g, &h);           // axisymmetric: no azimuth
+        // (axisymmetric: no azimuth)
+        if(FAST) evalCells<6, EVAL_AXI>(M, R, z, 1, 0, &Phi, &g, &h);
+        else     evalCellsCyl<6, EVAL_AXI>(M, R, z, 0, &Phi, &g, &h);
     }
-    __device__ double equatorial(const MultipoleView& M, double rsq) { return Phi0 = potentialOnAxes(M, rsq, 0); }
+    __device__ double onAxes(double rsq, int axis)
+    {
+        if(!FAST) return potentialOnAxes(*view, rsq, axis);
+        if(inCells(*view, rsq)) return cellsOnAxes(*view, rsq, axis);
+        const double r = sqrt(rsq);
+        double v, unused;
+        powerLawAxi<false>(rsq < view->rInnerSq ? view->inner : view->outer, rsq, axis ? 0 : r, axis ? r : 0, &v, &unused,
+            &unused);
+        return v;
+    }
+    __device__ double equatorial(double rsq) { return Phi0 = onAxes(rsq, 0); }
     __device__ FudgeBranch branch(bool lambdaBranch) const
     {
         FudgeBranch f;
@@ -318,18 +377,24 @@ struct CellPoint {
         fudgeSecond(rec->E, rec->I3 - rec->fnu, rec->Lz * rec->Lz / 2, rec->D2, fabs(rec->nu), rec->lambda, R, z, Phi,
             g, h, v, d, d2);
     }
-    __device__ void secondAt(double tau, double* v, double* d, double* d2) const
+    __device__ void secondAt(double tau, double* v, double* d, double* d2)
     {
-        fudgeSecondAt(*view, branch(true), tau, v, d, d2);
+        if(FAST) { rare = true; *v = *d = *d2 = NAN; }
+        else fudgeSecondAt(*view, branch(true), tau, v, d, d2);
     }
-    __device__ double nuValue(double tau) const { return fudgeValueAt(*view, branch(false), tau); }
-    __device__ double lambdaValue(double tau) const { return fudgeValueAt(*view, branch(true), tau); }
+    __device__ double valueAt(bool lambdaBranch, double tau)
+    {
+        if(FAST) { rare = true; return NAN; }
+        return fudgeValueAt(*view, branch(lambdaBranch), tau);
+    }
+    __device__ double nuValue(double tau) { return valueAt(false, tau); }
+    __device__ double lambdaValue(double tau) { return valueAt(true, tau); }
     // at Delta^2, on the axis (R = 0, z = sqrt(nu)): F needs no potential, F' its value alone
-    __device__ void endD2(double* v, double* d) const
+    __device__ void endD2(double* v, double* d)
     {
         const double n = fabs(rec->nu), D2 = rec->D2, L2h = rec->Lz * rec->Lz / 2;
         *v = -L2h * D2;
-        *d = rec->E * D2 - L2h - (rec->I3 - rec->fnu) - (D2 - n) * potentialOnAxes(*view, n, 1);
+        *d = rec->E * D2 - L2h - (rec->I3 - rec->fnu) - (D2 - n) * onAxes(n, 1);
     }
     // at |nu|, on the nu branch: the point itself
     __device__ void endNu(double* v, double* d) const
@@ -346,7 +411,8 @@ struct CellPoint {
     brackets go into the record; limits that need no root are stored directly (NaN otherwise).
     ends receives F and F' at the ends of the plain brackets (FudgeEnds), which the
     root searches then take instead of evaluating them. */
-static __device__ __forceinline__ void fudgeLimitsSetup(const CellPoint& fnc, FudgeRecord& rec, FudgeEnds* ends)
+template<bool FAST>
+static __device__ __forceinline__ void fudgeLimitsSetup(CellPoint<FAST>& fnc, FudgeRecord& rec, FudgeEnds* ends)
 {
     const double delta = rec.D2, lambda = rec.lambda;
     const double f_zero = fnc.zero();
@@ -428,10 +494,11 @@ static __device__ FudgeLimits fudgeLimitsFinish(const FudgeRecord& rec)
     stretch (integrateGL of ScaledIntegrand<ScalingCub>(AxisymIntegrand), src/math_core.cpp:1191-1205,
     src/actions_staeckel.cpp:276-299) at tau = lo + (hi - lo) s^2 (3 - 2 s): the integrand alone (the
     node's weight and du/ds / (hi - lo) come tabulated). */
+template<bool CELLS>
 __device__ __forceinline__ double fudgeMomentum(const MultipoleView& M, const FudgeBranch& f, double tau)
 {
     const double tmd = tau - f.D2;
-    const double p2 = f.value(M, tau) * rcpNormal(2 * pow2(tmd) * tau);
+    const double p2 = f.value<CELLS>(M, tau) * rcpNormal(2 * pow2(tmd) * tau);
     // p^2 < 0, NaN or infinite (a node on an end of the interval): no contribution
     return p2 > 1e-280 && p2 < INFINITY ? p2 * rsqrtNormal(p2) : 0;
 }
@@ -440,9 +507,10 @@ __device__ __forceinline__ double fudgeMomentum(const MultipoleView& M, const Fu
     quadrature): F(tau) and the point tau come from FP64 (the potential and the cancellation in
     F stay FP64), then p = sqrt(F / (2 tau)) / |tau - D2| is FP32 (the square root through the hardware
     reciprocal square root); the caller accumulates the weighted terms with compensation. */
+template<bool CELLS>
 __device__ __forceinline__ float fudgeMomentum32(const MultipoleView& M, const FudgeBranch& f, double tau)
 {
-    const double F = f.value(M, tau), tmd64 = tau - f.D2;
+    const double F = f.value<CELLS>(M, tau), tmd64 = tau - f.D2;
     // p = sqrt(F / (2 tau)) / |tau - D2|: the square root before the division by (tau - D2)^2
     // keeps every FP32 intermediate in range for tau up to ~1e18 (the product (tau - D2)^2 tau
     // overflows FP32 already at tau ~ 1e12, where loosely bound orbits reach); a value of F
@@ -459,12 +527,12 @@ __device__ __forceinline__ float fudgeMomentum32(const MultipoleView& M, const F
 
 /** Phase 1 of the actions of one point (R, z, phi, vR, vz, vphi) for focal distance fd
     (evalAxisymFudge, src/actions_staeckel.cpp:683-693: fd <= 0 falls back to max(R,1)*1e-4);
-    p has been located at the point.  Out of line, like locate(): one copy for
-    the kernels of given and of tabulated focal distances, so that both give the same bits.  Writes Jphi into act[2]; for a point without actions
+    p has been located at the point.  Writes Jphi into act[2]; for a point without actions
     (unbound, or lambda = nu = Delta^2) also NaN into act[0..1] and marks the record invalid.
     Otherwise the record holds the integrals of motion (findIntegralsOfMotionAxisymFudge,
     :176-195) and the limits and root brackets of fudgeLimitsSetup (ends: as there). */
-static __device__ __noinline__ void fudgePrepare(const MultipoleView& M, const double* pc, CellPoint& p, double fd,
+template<bool FAST>
+static __device__ __forceinline__ void fudgePrepare(const double* pc, CellPoint<FAST>& p, double fd,
     FudgeRecord& rec, double* act, FudgeEnds* ends)
 {
     const double Phi = p.Phi;
@@ -488,7 +556,7 @@ static __device__ __noinline__ void fudgePrepare(const MultipoleView& M, const d
     double absnu = 2 * D2 / (sum + sqD) * z2;
     if(absnu * 2 > D2) absnu = D2 - dmn; else dmn = D2 - absnu;
     if(sqD == 0) { act[0] = act[1] = NAN; return; }   // lambda = nu = Delta^2: undefined
-    const double Phi0 = p.equatorial(M, lambda - D2);
+    const double Phi0 = p.equatorial(lambda - D2);
     const double Ekin = 0.5 * (vR * vR + vz * vz + vphi * vphi);
     rec.lambda = lambda; rec.nu = absnu * signz; rec.D2 = D2; rec.E = Phi + Ekin; rec.Lz = Lz; rec.phi = phi;
     rec.flambda = -lambda * Phi0;
@@ -504,17 +572,19 @@ static __device__ __noinline__ void fudgePrepare(const MultipoleView& M, const d
         (nudot < 0 ? REC_NUDOT_NEG : 0);
 }
 
-/// Cartesian posvel -> cylindrical (R, z, phi, vR, vz, vphi); reference src/coord.cpp:476-484
+/// Cartesian posvel -> cylindrical (R, z, phi, vR, vz, vphi); reference src/coord.cpp:476-484; without
+/// AZIMUTH phi is left 0 (only the angles need it)
+template<bool AZIMUTH>
 __device__ __forceinline__ void carToCylPosVel(const double* w, double* pc)
 {
     const double R = sqrt(w[0] * w[0] + w[1] * w[1]);
     if(R == 0) {
-        pc[0] = 0; pc[1] = w[2]; pc[2] = atan2(w[4], w[3]);
+        pc[0] = 0; pc[1] = w[2]; pc[2] = AZIMUTH ? atan2(w[4], w[3]) : 0;
         pc[3] = sqrt(w[3] * w[3] + w[4] * w[4]); pc[4] = w[5]; pc[5] = 0;
         return;
     }
     const double c = w[0] / R, s = w[1] / R;
-    pc[0] = R; pc[1] = w[2]; pc[2] = atan2(w[1], w[0]);
+    pc[0] = R; pc[1] = w[2]; pc[2] = AZIMUTH ? atan2(w[1], w[0]) : 0;
     pc[3] = w[3] * c + w[4] * s;
     pc[4] = w[5];
     pc[5] = -w[3] * s + w[4] * c;

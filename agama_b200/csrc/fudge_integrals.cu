@@ -36,9 +36,12 @@ struct WarpIntegrals {
     the order of the nodes, when its last one is done, so the result does not depend on which
     integrals share a warp.
     MIXED: the integrand's arithmetic after F(tau) in FP32 (fudgeMomentum32) and the weighted
-    terms summed in FP32 with a compensation term (Kahan), converted to FP64 at the end. */
-template<bool MIXED>
-__global__ void __launch_bounds__(INTEGRAL_BLOCK, 4) fudgeIntegralKernel(const __grid_constant__ MultipoleView M,
+    terms summed in FP32 with a compensation term (Kahan), converted to FP64 at the end.
+    CELLS: the potential has cells.
+    Bound by the latency of its FP64 chains and of the L1: 1e6 disk points at 3 / 4 / 5 / 6 / 7 / 8 blocks per
+    SM 687 / 580 / 508 / 484 / 471 / 470 us, 7e5 halo points 716 / 630 / 550 / 533 / 528 / 533. */
+template<bool MIXED, bool CELLS>
+__global__ void __launch_bounds__(INTEGRAL_BLOCK, 7) fudgeIntegralKernel(const __grid_constant__ MultipoleView M,
     const __grid_constant__ GLRules gl, long n, int points, const FudgeRecord* __restrict__ rec,
     double* __restrict__ act, unsigned long long* __restrict__ counter)
 {
@@ -97,8 +100,8 @@ __global__ void __launch_bounds__(INTEGRAL_BLOCK, 4) fudgeIntegralKernel(const _
                 f.lam = j < static_cast<int>(lambdaSlots);
                 const double2 g = ldg2(W.rule[j] + 2 * (node - W.start[j]));
                 const double tau = fma(W.width[j], g.x, W.lo[j]);
-                W.term[node & 127] = MIXED ? static_cast<double>(static_cast<float>(g.y) * fudgeMomentum32(M, f, tau))
-                                           : g.y * fudgeMomentum(M, f, tau);
+                W.term[node & 127] = MIXED ? static_cast<double>(static_cast<float>(g.y) * fudgeMomentum32<CELLS>(M, f, tau))
+                                           : g.y * fudgeMomentum<CELLS>(M, f, tau);
             }
             __syncwarp();
             if(mine && end > base && end <= base + 32) {        // (at most 40 + 32 nodes back: in the ring)
@@ -122,7 +125,7 @@ __global__ void __launch_bounds__(INTEGRAL_BLOCK, 4) fudgeIntegralKernel(const _
 }
 
 /// resident blocks of the integral kernel on the current device (cached per device and variant)
-template<bool MIXED>
+template<bool MIXED, bool CELLS>
 int integralGridSize()
 {
     static std::mutex mutex;
@@ -134,7 +137,7 @@ int integralGridSize()
     if(it != cache.end()) return it->second;
     int sms = 0, perSM = 0;
     AGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    AGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, fudgeIntegralKernel<MIXED>, INTEGRAL_BLOCK, 0));
+    AGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, fudgeIntegralKernel<MIXED, CELLS>, INTEGRAL_BLOCK, 0));
     const int grid = std::max(1, sms * std::max(1, perSM));
     cache[dev] = grid;
     return grid;
@@ -142,20 +145,30 @@ int integralGridSize()
 
 }  // namespace
 
-void launchFudgeIntegrals(const MultipoleView& M, const GLRules& gl, long n, const FudgeRecord* rec, double* act,
-    unsigned long long* counter, bool mixed, cudaStream_t stream)
+namespace {
+template<bool MIXED, bool CELLS>
+void launchIntegrals(const MultipoleView& M, const GLRules& gl, long n, const FudgeRecord* rec, double* act,
+    unsigned long long* counter, cudaStream_t stream)
 {
-    if(n <= 0) return;
-    AGB_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), stream));
-    const long resident = mixed ? integralGridSize<true>() : integralGridSize<false>();
+    const long resident = integralGridSize<MIXED, CELLS>();
     // 16 points a claim, fewer where that would leave warps without any
     int points = 16;
     while(points > 1 && n < points * resident * WARPS_PER_BLOCK) points /= 2;
     const long claims = (n + points - 1) / points;
     const long grid = std::min(resident, (claims + WARPS_PER_BLOCK - 1) / WARPS_PER_BLOCK);
-    (mixed ? fudgeIntegralKernel<true> : fudgeIntegralKernel<false>)<<<grid, INTEGRAL_BLOCK, 0, stream>>>(M, gl, n,
-        points, rec, act, counter);
+    fudgeIntegralKernel<MIXED, CELLS><<<grid, INTEGRAL_BLOCK, 0, stream>>>(M, gl, n, points, rec, act, counter);
     AGB_CUDA(cudaGetLastError());
+}
+}  // namespace
+
+void launchFudgeIntegrals(const MultipoleView& M, const GLRules& gl, long n, const FudgeRecord* rec, double* act,
+    unsigned long long* counter, bool mixed, cudaStream_t stream)
+{
+    if(n <= 0) return;
+    AGB_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), stream));
+    auto launch = M.cells ? (mixed ? launchIntegrals<true, true> : launchIntegrals<false, true>)
+                          : (mixed ? launchIntegrals<true, false> : launchIntegrals<false, false>);
+    launch(M, gl, n, rec, act, counter, stream);
 }
 
 }  // namespace agb

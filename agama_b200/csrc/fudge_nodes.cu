@@ -22,7 +22,7 @@ __global__ void __launch_bounds__(PREPARE_BLOCK, 5) nodePrepareKernel(const __gr
     if(i >= n) return;
     double w[6], pc[6];
     for(int c = 0; c < 6; c++) w[c] = posvel[6 * i + c];
-    carToCylPosVel(w, pc);
+    carToCylPosVel<true>(w, pc);
     double Phi;
     CylDerivs g; CylHess h;
     evalMultipoleCylCall<1, EVAL_AXI>(M, pc[0], pc[1], 0, &Phi, &g, &h);   // axisymmetric: no azimuth

@@ -104,9 +104,11 @@ __device__ __forceinline__ bool predictedBracket(const FudgeRecord& r, int kind,
     iterations} when STATS.  LEARNED = false (no predictions, no stats) compiles the plain searches
     alone, without that state and the counters (fewer registers); STATS = false leaves the
     counters out of the learned searches.  NODES = true evaluates F from the node form of the splines
-    (points whose angles follow), false from the cells. */
+    (points whose angles follow, potentials without cells), false from the cells: without a call in the
+    evaluation the searches fit 80 registers (1e6 disk points at 3 / 4 / 5 / 6 / 7 / 8 blocks per SM 1265 / 1015 /
+    930 / 908 / 945 / 1040 us; with the call and 370 B of spills 1150 at 4). */
 template<bool LEARNED, bool STATS, bool NODES>
-__global__ void __launch_bounds__(ROOT_BLOCK, 4) fudgeRootKernel(const __grid_constant__ MultipoleView M, long n,
+__global__ void __launch_bounds__(ROOT_BLOCK, NODES ? 4 : 6) fudgeRootKernel(const __grid_constant__ MultipoleView M, long n,
     FudgeRecord* __restrict__ rec, const FudgeEnds* __restrict__ ends, int* __restrict__ iters,
     unsigned long long* __restrict__ counter, const float* __restrict__ pred, const BracketWidths widths,
     unsigned long long* __restrict__ stats)
@@ -233,7 +235,7 @@ __global__ void __launch_bounds__(ROOT_BLOCK, 4) fudgeRootKernel(const __grid_co
         double fx = 0, dx = 0;
         if(mode == LANE_EVAL || mode == LANE_VERIFY) {
             if constexpr(NODES) limitRootEval(fnc, kind, u0, x, &fx, &dx);
-            else limitRootEval(M, fnc, kind == ROOT_LAMBDA_MAX, u0, x, &fx, &dx);
+            else limitRootEval<true>(M, fnc, kind == ROOT_LAMBDA_MAX, u0, x, &fx, &dx);
         }
         // 4. the values fed to the searches
         if(mode == LANE_EVAL) {

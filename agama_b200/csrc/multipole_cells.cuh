@@ -114,18 +114,21 @@ __device__ __forceinline__ void cellPolynomial(const double* __restrict__ c, dou
     if(NQ == 6) { *pss = 2 * vss; *pst = vst; *ptt = 2 * vtt; }
 }
 
+/// value, gradient and Hessian of an evaluation out of line
+struct BeyondCells { double pot; CylDerivs g; CylHess h; };
+
 /// the rare places: the asymptotic expansions beyond the radial grid, the 1-D splines of lmax <= 2
 /// and 2-D splines without cells; out of line so that the callers' registers and
-/// instruction stream are those of the cells
+/// instruction stream are those of the cells (the callers copy from a result of this branch's own: one
+/// whose address left the common path would keep the common results in local memory)
 template<int NQ>
-__device__ __noinline__ void evalBeyondCells(const MultipoleView& M, double R, double z, double phi,
-    double* pot, CylDerivs* g, CylHess* h)
+__device__ __noinline__ void evalBeyondCells(const MultipoleView& M, double R, double z, double phi, BeyondCells* r)
 {
     const double rsq = R * R + z * z;
-    if(rsq < M.rInnerSq)      evalPowerLaw<NQ>(M.inner, R, z, phi, pot, g, h);
-    else if(rsq > M.rOuterSq) evalPowerLaw<NQ>(M.outer, R, z, phi, pot, g, h);
-    else if(M.is2d)           evalInterp2d<NQ>(M, R, z, phi, pot, g, h);
-    else                      evalInterp1d<NQ>(M, R, z, phi, pot, g, h);
+    if(rsq < M.rInnerSq)      evalPowerLaw<NQ>(M.inner, R, z, phi, &r->pot, &r->g, &r->h);
+    else if(rsq > M.rOuterSq) evalPowerLaw<NQ>(M.outer, R, z, phi, &r->pot, &r->g, &r->h);
+    else if(M.is2d)           evalInterp2d<NQ>(M, R, z, phi, &r->pot, &r->g, &r->h);
+    else                      evalInterp1d<NQ>(M, R, z, phi, &r->pot, &r->g, &r->h);
 }
 
 /** The 2-D spline evaluation (MultipoleInterp2d::evalCyl, src/potential_multipole.cpp:1969-2080) from
@@ -241,8 +244,13 @@ __device__ __forceinline__ void evalCellsCyl(const MultipoleView& M, double R, d
         double sphi = 0, cphi = 1;
         if(KIND == EVAL_FAST) sincos(phi, &sphi, &cphi);
         evalCells<NQ, KIND>(M, R, z, cphi, sphi, pot, g, h);
-    } else
-        evalBeyondCells<NQ>(M, R, z, phi, pot, g, h);
+    } else {
+        BeyondCells r;
+        evalBeyondCells<NQ>(M, R, z, phi, &r);
+        *pot = r.pot;
+        if(NQ >= 3) *g = r.g;
+        if(NQ == 6) *h = r.h;
+    }
 }
 
 /** Evaluation at a Cartesian point with gradient (and Hessian xx,yy,zz,xy,yz,zx) in Cartesian
@@ -259,8 +267,13 @@ __device__ __forceinline__ void evalCellsCar(const MultipoleView& M, double x, d
     CylDerivs g; CylHess h;
     if(inCells(M, R * R + z * z))
         evalCells<NQ, KIND>(M, R, z, axis ? 1 : c, s, pot, &g, &h);
-    else
-        evalBeyondCells<NQ>(M, R, z, axis ? 0 : atan2(y, x), pot, &g, &h);
+    else {
+        BeyondCells r;
+        evalBeyondCells<NQ>(M, R, z, axis ? 0 : atan2(y, x), &r);
+        *pot = r.pot;
+        if(NQ >= 3) g = r.g;
+        if(NQ == 6) h = r.h;
+    }
     if(NQ == 1) return;
     // on the axis the transformation is degenerate: the derivatives of R and phi are given as 1
     const double dRdx = axis ? 1 : c, dRdy = axis ? 1 : s, dphidx = axis ? 1 : -s * Rinv, dphidy = axis ? 1 : c * Rinv;

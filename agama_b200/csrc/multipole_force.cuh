@@ -450,8 +450,13 @@ __device__ __forceinline__ void evalForceCar(const MultipoleView& M, double x, d
         evalMultipoleCyl<3, KIND>(M, R, z, phi, pot, &g, &h);
     } else if(inCells(M, rsq))
         forceInterp2d<KIND, G, MIXED>(M, R, z, phi, pot, &g);
-    else
-        forceBeyond(M, R, z, phi, pot, &g);
+    else {      // (results of this branch's own: the common ones stay in registers)
+        double p;
+        CylDerivs d;
+        forceBeyond(M, R, z, phi, &p, &d);
+        *pot = p;
+        g = d;
+    }
     grad[0] = noAzimuth ? g.dR * dRdx : sumProducts(g.dR, dRdx, g.dphi, dphidx);
     grad[1] = noAzimuth ? g.dR * dRdy : sumProducts(g.dR, dRdy, g.dphi, dphidy);
     grad[2] = g.dz;
