@@ -164,20 +164,21 @@ class Potential:
             out.append(hess[0] if single else hess)
         return out[0] if len(out) == 1 else tuple(out)
 
-    def _eval_device(self, points, pot, acc, der):
+    def _eval_device(self, points, pot, acc, der, negate=False):
+        """negate: the derivatives of the acceleration instead of the Hessian"""
         import torch
         p = points.contiguous().view(-1, 3)
         n = p.shape[0]
-        phi = torch.empty(n, dtype=torch.float64, device=p.device)
-        grad = torch.empty((n, 3), dtype=torch.float64, device=p.device) if (acc or der) else None
+        phi = torch.empty(n, dtype=torch.float64, device=p.device) if pot or not (acc or der) else None
+        grad = torch.empty((n, 3), dtype=torch.float64, device=p.device) if acc else None
         hess = torch.empty((n, 6), dtype=torch.float64, device=p.device) if der else None
-        check(_native.lib().agama_evalPotentialManyDevice(
-            self._h, n, _dev_ptr(p), _dev_ptr(phi), _dev_ptr(grad), _dev_ptr(hess), _current_stream()))
+        check(_native.lib().agama_evalAccelerationManyDevice(
+            self._h, n, _dev_ptr(p), _dev_ptr(phi), _dev_ptr(grad), _dev_ptr(hess), 1 if negate else 0, _current_stream()))
         out = []
         if pot:
             out.append(phi)
         if acc:
-            out.append(-grad)
+            out.append(grad)
         if der:
             out.append(hess)
         return out[0] if len(out) == 1 else tuple(out)
@@ -200,6 +201,8 @@ class Potential:
 
     def forceDeriv(self, points):
         """force and the derivatives of force (= minus the Hessian), as agama's forceDeriv"""
+        if _is_device_array(points):
+            return self._eval_device(points, False, True, True, negate=True)
         f, h = self.eval(points, pot=False, acc=True, der=True)
         return f, -h
 

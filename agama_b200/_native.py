@@ -31,6 +31,7 @@ SIGNATURES = {
     "agama_writeMultipoleCoefs": (ctypes.c_int, [ctypes.c_char_p, ctypes.c_int, D, ctypes.c_int, D, D]),
     "agama_evalPotentialMany": (ctypes.c_int, [VP, ctypes.c_long, D, ctypes.c_double, D, D, D]),
     "agama_evalPotentialManyDevice": (ctypes.c_int, [VP, ctypes.c_long, VP, VP, VP, VP, VP]),
+    "agama_evalAccelerationManyDevice": (ctypes.c_int, [VP, ctypes.c_long, VP, VP, VP, VP, ctypes.c_int, VP]),
     "agama_evalPotentialCylMany": (ctypes.c_int, [VP, ctypes.c_long, D, ctypes.c_double, D, D, D]),
     "agama_evalPotentialCylManyDevice": (ctypes.c_int, [VP, ctypes.c_long, VP, VP, VP, VP, VP]),
     "agama_createDensity": (VP, [ctypes.c_char_p]),

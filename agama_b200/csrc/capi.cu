@@ -214,6 +214,17 @@ int agama_evalPotentialManyDevice(const agama_Potential* p, long n, const double
     });
 }
 
+int agama_evalAccelerationManyDevice(const agama_Potential* p, long n, const double* pos,
+    double* phi, double* acc, double* deriv2, int negateDeriv2, void* stream)
+{
+    return guarded([&] {
+        if(!p || n < 0 || (n > 0 && !pos)) throw std::invalid_argument("evalAccelerationManyDevice: invalid arguments");
+        AGB_CUDA(cudaSetDevice(p->pot->device));
+        launchEvalPotential(p->pot->view, n, pos, phi, acc, deriv2, static_cast<cudaStream_t>(stream), false, -1,
+            negateDeriv2 ? -1 : 1);
+    });
+}
+
 int agama_evalPotentialMany(const agama_Potential* p, long n, const double* pos, double time,
     double* phi, double* deriv, double* deriv2)
 {

@@ -253,28 +253,29 @@ __device__ __forceinline__ void evalCellsCyl(const MultipoleView& M, double R, d
     }
 }
 
+/// a Cartesian point beyond the cells (or of a potential without them), out of line
+template<int NQ>
+__device__ __noinline__ void evalBeyondCellsCar(const MultipoleView& M, double x, double y, double z, double* pot,
+    double* grad, double* hess)
+{
+    evalMultipoleCar<NQ, EVAL_GENERAL>(M, x, y, z, pot, grad, hess);
+}
+
 /** Evaluation at a Cartesian point with gradient (and Hessian xx,yy,zz,xy,yz,zx) in Cartesian
-    coordinates, as evalMultipoleCar: inside the cells the azimuth enters only through its cosine and
-    sine, x / R and y / R, so neither atan2 nor sincos is formed. */
+    coordinates, as evalMultipoleCar: the azimuth enters only through its cosine and
+    sine, x / R and y / R, so neither atan2 nor sincos is formed.  False for a point beyond the cells
+    (nothing evaluated). */
 template<int NQ, int KIND>
-__device__ __forceinline__ void evalCellsCar(const MultipoleView& M, double x, double y, double z,
+__device__ __forceinline__ bool evalCellsCar(const MultipoleView& M, double x, double y, double z,
     double* pot, double* grad, double* hess)
 {
-    if(KIND == EVAL_GENERAL) { evalMultipoleCar<NQ, KIND>(M, x, y, z, pot, grad, hess); return; }
     const double R2 = x * x + y * y, R = sqrt(R2);
+    if(!inCells(M, R * R + z * z)) return false;
     const bool axis = R == 0;
     const double Rinv = axis ? 0 : 1 / R, c = x * Rinv, s = y * Rinv;
     CylDerivs g; CylHess h;
-    if(inCells(M, R * R + z * z))
-        evalCells<NQ, KIND>(M, R, z, axis ? 1 : c, s, pot, &g, &h);
-    else {
-        BeyondCells r;
-        evalBeyondCells<NQ>(M, R, z, axis ? 0 : atan2(y, x), &r);
-        *pot = r.pot;
-        if(NQ >= 3) g = r.g;
-        if(NQ == 6) h = r.h;
-    }
-    if(NQ == 1) return;
+    evalCells<NQ, KIND>(M, R, z, axis ? 1 : c, s, pot, &g, &h);
+    if(NQ == 1) return true;
     // on the axis the transformation is degenerate: the derivatives of R and phi are given as 1
     const double dRdx = axis ? 1 : c, dRdy = axis ? 1 : s, dphidx = axis ? 1 : -s * Rinv, dphidy = axis ? 1 : c * Rinv;
     grad[0] = g.dR * dRdx + g.dphi * dphidx;
@@ -296,6 +297,7 @@ __device__ __forceinline__ void evalCellsCar(const MultipoleView& M, double x, d
         hess[4] = h.dRdz * dRdy + h.dzdphi * dphidy;                                          // yz
         hess[5] = h.dRdz * dRdx + h.dzdphi * dphidx;                                          // zx
     }
+    return true;
 }
 
 }  // namespace agb

@@ -12,22 +12,34 @@ thread_local std::string g_error;
 /// KIND = spline evaluator matching the potential (EvalKind).  Bound by the L1: each lane reads its own
 /// cells, nine 32-byte loads a harmonic at one data-stage cycle per lane (60 % of its rate at 2e6
 /// points of the triaxial lmax 6 potential, value and gradient: 543 us from the node form at 168
-/// registers, 410 from the cells with 16-byte loads at 80 registers, 330 with 32-byte loads; with
-/// the Hessian and the density at 4e5 points 294 -> 174 us).
+/// registers, 410 from the cells with 16-byte loads at 80 registers, 330 with 32-byte loads, 305 with the
+/// sign applied here instead of in a pass of its own; with the Hessian and the density at 4e5 points 294 -> 174 -> 163 us).
+/// gradSign, hessSign: 1, or -1 for the acceleration and its derivatives.
 template<int NQ, int KIND>
 __global__ void __launch_bounds__(128, NQ == 6 ? 4 : 6) evalPotentialKernel(const __grid_constant__ MultipoleView M, long n,
     const double* __restrict__ pos, double* __restrict__ phi, double* __restrict__ grad,
-    double* __restrict__ hess)
+    double* __restrict__ hess, double gradSign, double hessSign)
 {
     const long i = blockIdx.x * static_cast<long>(blockDim.x) + threadIdx.x;
     if(i >= n) return;
     const double x = pos[3 * i], y = pos[3 * i + 1], z = pos[3 * i + 2];
-    double p, g[3], h[6];
-    evalCellsCar<NQ, KIND>(M, x, y, z, &p, g, h);
-    if(phi) phi[i] = p;
-    if(NQ >= 3 && grad) { grad[3 * i] = g[0]; grad[3 * i + 1] = g[1]; grad[3 * i + 2] = g[2]; }
-    if(NQ == 6 && hess)
-        for(int k = 0; k < 6; k++) hess[6 * i + k] = h[k];
+    auto store = [&](double p, const double* g, const double* h) {
+        if(phi) phi[i] = p;
+        if(NQ >= 3 && grad)
+            for(int k = 0; k < 3; k++) grad[3 * i + k] = gradSign * g[k];
+        if(NQ == 6 && hess)
+            for(int k = 0; k < 6; k++) hess[6 * i + k] = hessSign * h[k];
+    };
+    if(KIND != EVAL_GENERAL) {
+        double p, g[3], h[6];
+        if(evalCellsCar<NQ, KIND == EVAL_GENERAL ? EVAL_AXI : KIND>(M, x, y, z, &p, g, h)) {
+            store(p, g, h);
+            return;
+        }
+    }
+    double p, g[3], h[6];       // (variables of the rare path's own: its call takes their addresses)
+    evalBeyondCellsCar<NQ>(M, x, y, z, &p, g, h);
+    store(p, g, h);
 }
 
 /// the same at n cylindrical points (R, z, phi), derivatives in cylindrical coordinates
@@ -150,7 +162,7 @@ void requireDevice()
 }
 
 void launchEvalPotential(const MultipoleView& M, long n, const double* pos, double* phi,
-    double* grad, double* hess, cudaStream_t stream, bool cylindrical)
+    double* grad, double* hess, cudaStream_t stream, bool cylindrical, double gradSign, double hessSign)
 {
     if(n <= 0) return;
     const int block = 128;
@@ -158,7 +170,7 @@ void launchEvalPotential(const MultipoleView& M, long n, const double* pos, doub
     const int nq = hess ? 6 : grad ? 3 : 1, kind = evalKindOf(M);
 #define AGB_LAUNCH(NQ_, K_) \
     (cylindrical ? evalPotentialCylKernel<NQ_, K_><<<grid, block, 0, stream>>>(M, n, pos, phi, grad, hess) \
-                 : evalPotentialKernel<NQ_, K_><<<grid, block, 0, stream>>>(M, n, pos, phi, grad, hess))
+                 : evalPotentialKernel<NQ_, K_><<<grid, block, 0, stream>>>(M, n, pos, phi, grad, hess, gradSign, hessSign))
     if(kind == EVAL_AXI)       { if(nq == 6) AGB_LAUNCH(6, EVAL_AXI);     else if(nq == 3) AGB_LAUNCH(3, EVAL_AXI);     else AGB_LAUNCH(1, EVAL_AXI); }
     else if(kind == EVAL_FAST) { if(nq == 6) AGB_LAUNCH(6, EVAL_FAST);    else if(nq == 3) AGB_LAUNCH(3, EVAL_FAST);    else AGB_LAUNCH(1, EVAL_FAST); }
     else                       { if(nq == 6) AGB_LAUNCH(6, EVAL_GENERAL); else if(nq == 3) AGB_LAUNCH(3, EVAL_GENERAL); else AGB_LAUNCH(1, EVAL_GENERAL); }

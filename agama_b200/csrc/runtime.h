@@ -82,9 +82,10 @@ DeviceActionFinder* createDeviceActionFinder(DevicePotential* pot, const FinderT
 FinderTablesHost buildFinderTables(const DevicePotential& P);
 
 /// launch helpers (defined in the .cu files)
-/// (cylindrical: points (R, z, phi) and derivatives in cylindrical coordinates)
+/// (cylindrical: points (R, z, phi) and derivatives in cylindrical coordinates; gradSign, hessSign:
+/// factors 1 or -1 of the Cartesian derivatives)
 void launchEvalPotential(const MultipoleView& M, long n, const double* pos, double* phi,
-    double* grad, double* hess, cudaStream_t stream, bool cylindrical = false);
+    double* grad, double* hess, cudaStream_t stream, bool cylindrical = false, double gradSign = 1, double hessSign = 1);
 /// density (Laplacian / 4 pi inside the grid, closed form outside) at n Cartesian points
 void launchDensity(const MultipoleView& M, long n, const double* pos, double* rho, cudaStream_t stream);
 /// radius queries in the equatorial plane of the azimuthally averaged potential: a = E (or L for

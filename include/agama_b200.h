@@ -140,6 +140,12 @@ int agama_evalPotentialMany(const agama_Potential* potential, long n, const doub
 int agama_evalPotentialManyDevice(const agama_Potential* potential, long n, const double* pos,
     double* phi, double* deriv, double* deriv2, void* stream);
 
+/* The same with the acceleration (minus the gradient) in place of the gradient and, when negateDeriv2 is
+   not 0, its derivatives (minus the Hessian) in place of the Hessian: no pass over the results to
+   change their sign. */
+int agama_evalAccelerationManyDevice(const agama_Potential* potential, long n, const double* pos,
+    double* phi, double* acc, double* deriv2, int negateDeriv2, void* stream);
+
 /* Batched potential / gradient / Hessian at n cylindrical points, host buffers: pos is n x 3 in the
    order (R, z, phi) of the reference's coord::PosCyl; deriv n x 3 (dR, dz, dphi) as coord::GradCyl;
    deriv2 n x 6 (dR2, dz2, dphi2, dRdz, dzdphi, dRdphi) as coord::HessCyl.  Replaces n calls of
