@@ -221,29 +221,37 @@ AGB_HD double scaleCub(double ul, double ur, double u)
 // Root finder (reference src/math_core.cpp:866-1041: hybrid of Brent's method and a
 // monotone Hermite-interpolation step when derivatives are available)
 
+/// the divisions and roots of the root searches
+struct ExactArithmetic {
+    static AGB_HD double quotient(double a, double b) { return a / b; }
+    static AGB_HD double root(double a) { return sqrt(a); }
+};
+
 /// Hermite cubic through (x1,f1,d1), (x2,f2,d2) evaluated at x
+template<class A = ExactArithmetic>
 AGB_HD double hermiteCubic(double x, double x1, double x2, double f1, double f2, double d1, double d2)
 {
-    const double h = x2 - x1, t = (x - x1) / h, T = 1 - t;
+    const double h = x2 - x1, t = A::quotient(x - x1, h), T = 1 - t;
     return f1 * T * T * (1 + 2 * t) + f2 * t * t * (1 + 2 * T) + d1 * h * T * T * t - d2 * h * t * t * T;
 }
 
 /// the same, but NaN if the cubic is not monotone on [x1, x2]
+template<class A = ExactArithmetic>
 AGB_HD double hermiteMonotone(double x, double x1, double x2, double f1, double f2, double d1, double d2)
 {
     if(!isFinite(d1 + d2) || (d1 >= 0 && d2 < 0) || (d2 >= 0 && d1 < 0))
         return NAN;
     const double dx = x2 - x1;
-    const double ai = 1 / (-6 * (f2 - f1) / dx + 3 * (d1 + d2));
+    const double ai = A::quotient(1, A::quotient(-6 * (f2 - f1), dx) + 3 * (d1 + d2));
     const double ba = -1 + (d2 - d1) * ai, ca = d1 * ai, D = pow2(ba) - 4 * ca;
     if(!isFinite(ba + D))
         return NAN;
     if(D >= 0) {
-        const double sq = sqrt(D), t1 = 0.5 * (-ba - sq), t2 = 0.5 * (-ba + sq);
+        const double sq = A::root(D), t1 = 0.5 * (-ba - sq), t2 = 0.5 * (-ba + sq);
         if((t1 >= 0 && t1 <= 1) || (t2 >= 0 && t2 <= 1))
             return NAN;
     }
-    return hermiteCubic(x, x1, x2, f1, f2, d1, d2);
+    return hermiteCubic<A>(x, x1, x2, f1, f2, d1, d2);
 }
 
 constexpr int ROOT_MAXITER = 64;
@@ -343,7 +351,8 @@ AGB_HD double findRoot(const F& fnc, double xlower, double xupper, double reltol
         double x = s.start(lo, hi, reltol);
         while(true) { f(x, &fx, &dx); if(s.feed(fx, dx, &x)) break; }
         root = s.result; iterations = s.iter;                                               */
-struct RootSearch {
+template<class A>
+struct RootSearchOf {
     double a, b, c, fa, fb, fc, da, db, dc, d, e, abstol;
     double result;
     int iter, phase;     // phase 0: wants f(xlower), 1: f(xupper), 2: f(next iterate),
@@ -429,16 +438,12 @@ struct RootSearch {
             a = b; b = c; c = a;  fa = fb; fb = fc; fc = fa;  da = db; db = dc; dc = da;
         }
         iter++;
-        if(fabs(b - c) <= abstol) {
-            const double off = fb * (b - c) / (fc - fb);
-            if((off > 0 && off < c - b) || (off < 0 && off > c - b))
-                b += off;
-            result = b;
-            return 0;
-        }
-        const double off = -fb / db;
+        // the final secant step once the bracket is small enough, otherwise a Newton step within
+        // the bracket if that is small enough (one quotient for both)
+        const bool narrow = fabs(b - c) <= abstol;
+        const double off = A::quotient(narrow ? fb * (b - c) : -fb, narrow ? fc - fb : db);
         const bool inside = (off > 0 && off < c - b) || (off < 0 && off > c - b);
-        if(inside && fabs(off) < abstol) { result = b + off; return 0; }
+        if(narrow || (inside && fabs(off) < abstol)) { result = inside ? b + off : b; return 0; }
         if(iter >= ROOT_MAXITER) { result = b; return 0; }
         return 1;
     }
@@ -486,23 +491,23 @@ struct RootSearch {
         } else {
             double dd = NAN;
             if(db * dc > 0)
-                dd = hermiteMonotone(0, fb, fc, 0, cb, 1 / db, 1 / dc);
+                dd = hermiteMonotone<A>(0, fb, fc, 0, cb, A::quotient(1, db), A::quotient(1, dc));
             if(isFinite(dd) && fmin(fabs(dd), fabs(cb - dd)) > fabs(cb) * ROOT_DELTA_HERMITE) {
                 d = dd;
             } else {
-                double p, q, r, s = fb / fa;
+                double p, q, r, s = A::quotient(fb, fa);
                 if(a == c) {
                     p = 2 * m * s;
                     q = 1 - s;
                 } else {
-                    q = fa / fc;
-                    r = fb / fc;
+                    q = A::quotient(fa, fc);
+                    r = A::quotient(fb, fc);
                     p = s * (2 * m * q * (q - r) - (b - a) * (r - 1));
                     q = (q - 1) * (r - 1) * (s - 1);
                 }
                 if(p > 0) q = -q; else p = -p;
                 if(2 * p < fmin(3 * m * q - fabs(tol * q), fabs(e * q))) {
-                    e = d; d = p / q;
+                    e = d; d = A::quotient(p, q);
                 } else {
                     d = m; e = m;
                 }
@@ -514,5 +519,6 @@ struct RootSearch {
         return false;
     }
 };
+using RootSearch = RootSearchOf<ExactArithmetic>;
 
 }  // namespace agb

@@ -159,11 +159,11 @@ struct FudgeBranch {
         lam = lambdaBranch;
         E = E_; D2 = D2_; L2h = Lz * Lz / 2;
         I = lam ? I3 - fnu : I3 - flambda;
-        const double n = fabs(nu), lmd = lambda - D2, inv = 1 / D2;
+        const double n = fabs(nu), lmd = lambda - D2, inv = rcpNormal(D2);
         mo = lam ? n : lambda;
         ro = lam ? n : lmd;
-        c1 = sqrt(lam ? 1 - n * inv : lmd * inv);
-        c2 = sqrt((lam ? n : lambda) * inv);
+        c1 = NormalArithmetic::root(lam ? 1 - n * inv : lmd * inv);
+        c2 = NormalArithmetic::root((lam ? n : lambda) * inv);
     }
 
     /// F(tau), and with DER its derivative.  CELLS: the potential has cells (2-D splines), and beyond them

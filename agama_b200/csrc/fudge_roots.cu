@@ -15,9 +15,13 @@ namespace {
 
 constexpr int ROOT_BLOCK = 128;
 constexpr unsigned FULL_MASK = 0xffffffffu;
+/// idle lanes of a warp that wait for one another before they take new searches (the set-up, 2 roots, 5 quotients
+/// and 180 bytes of loads, then runs for several lanes at once): 1e6 disk points at 1 / 8 / 16 lanes 819 / 805 / 821 us
+constexpr int REFILL = 8;
 
 /// the limit found by a plain search (nu_max falls back to |nu| when the search found no root)
-__device__ __forceinline__ void storePlainLimit(FudgeRecord& r, int kind, const RootSearch& s, double u0)
+template<class A>
+__device__ __forceinline__ void storePlainLimit(FudgeRecord& r, int kind, const RootSearchOf<A>& s, double u0)
 {
     if(kind == ROOT_NU_MAX) r.nuMax = isFinite(s.result) ? s.result : fabs(r.nu);
     else if(kind == ROOT_LAMBDA_MIN) r.lambdaMin = s.result;
@@ -33,7 +37,8 @@ enum { LANE_IDLE = 0, LANE_PROPOSE = 1, LANE_EVAL = 2, LANE_VERIFY = 3 };
     evaluation either (limitRootEval's values there).  Returns LANE_IDLE when the search has
     finished at once (no sign change, or a root at an end), LANE_PROPOSE when both ends are known
     and the first iterate is due from RootSearch::propose, LANE_EVAL when *x is an end to evaluate. */
-__device__ __forceinline__ int setupPlain(RootSearch& s, int kind, const FudgeEnds* e, double lo, double hi,
+template<class A>
+__device__ __forceinline__ int setupPlain(RootSearchOf<A>& s, int kind, const FudgeEnds* e, double lo, double hi,
     double tol, double u0, double D2, double E, double* x)
 {
     if(!e) { *x = s.startAbs(lo, hi, tol); return LANE_EVAL; }
@@ -48,7 +53,8 @@ __device__ __forceinline__ int setupPlain(RootSearch& s, int kind, const FudgeEn
         *x = s.startKnownUpper(lo, hi, tol, e->fPos, e->dfPos);
         return LANE_EVAL;
     }
-    const double fa = e->fPos / pow2(u0), da = (e->dfPos - 2 * e->fPos / u0) / pow2(u0) * u0;
+    const double fa = A::quotient(e->fPos, pow2(u0)),
+        da = A::quotient(e->dfPos - A::quotient(2 * e->fPos, u0), pow2(u0)) * u0;
     return s.setupKnownEnds(lo, hi, tol, fa, da, E, NAN) ? LANE_IDLE : LANE_PROPOSE;
 }
 
@@ -106,9 +112,12 @@ __device__ __forceinline__ bool predictedBracket(const FudgeRecord& r, int kind,
     counters out of the learned searches.  NODES = true evaluates F from the node form of the splines
     (points whose angles follow, potentials without cells), false from the cells: without a call in the
     evaluation the searches fit 80 registers (1e6 disk points at 3 / 4 / 5 / 6 / 7 / 8 blocks per SM 1265 / 1015 /
-    930 / 908 / 945 / 1040 us; with the call and 370 B of spills 1150 at 4). */
+    930 / 908 / 945 / 1040 us; with the call and 370 B of spills 1150 at 4).  Quotients and roots of the
+    searches' steps without the library's slow paths (NormalArithmetic): 919 -> 819 us, 366 B of spills; at 4 / 5 / 6 blocks
+    869 / 812 / 805 us.  The learned searches hold more state: 4 blocks (2417 us a step with the counters, 2562 at 6).
+    Bound by latency and issue together: 60 % of the issue slots, 19 of 32 lanes (the branches of a step). */
 template<bool LEARNED, bool STATS, bool NODES>
-__global__ void __launch_bounds__(ROOT_BLOCK, NODES ? 4 : 6) fudgeRootKernel(const __grid_constant__ MultipoleView M, long n,
+__global__ void __launch_bounds__(ROOT_BLOCK, NODES || LEARNED ? 4 : 6) fudgeRootKernel(const __grid_constant__ MultipoleView M, long n,
     FudgeRecord* __restrict__ rec, const FudgeEnds* __restrict__ ends, int* __restrict__ iters,
     unsigned long long* __restrict__ counter, const float* __restrict__ pred, const BracketWidths widths,
     unsigned long long* __restrict__ stats)
@@ -122,7 +131,7 @@ __global__ void __launch_bounds__(ROOT_BLOCK, NODES ? 4 : 6) fudgeRootKernel(con
     double x = 0, u0 = 0, verified = 0;
     unsigned nSearch = 0, nSeeded = 0, nFallback = 0, nIter = 0;
     std::conditional_t<NODES, FudgeFunction, FudgeBranch> fnc{};
-    RootSearch s;
+    RootSearchOf<std::conditional_t<NODES, ExactArithmetic, NormalArithmetic>> s;
     // a plain search on the point's bracket again (after a seeded root failed its check)
     auto restartPlain = [&]() {
         const FudgeRecord& r = rec[point];
@@ -164,7 +173,7 @@ __global__ void __launch_bounds__(ROOT_BLOCK, NODES ? 4 : 6) fudgeRootKernel(con
         //    sets it up
         while(true) {
             const unsigned need = __ballot_sync(FULL_MASK, mode == LANE_IDLE && !drained);
-            if(!need) break;
+            if(!need || (__popc(need) < REFILL && __any_sync(FULL_MASK, mode != LANE_IDLE))) break;
             const int leader = __ffs(need) - 1;
             unsigned long long base = 0;
             if(static_cast<int>(lane) == leader) base = atomicAdd(counter, static_cast<unsigned long long>(__popc(need)));

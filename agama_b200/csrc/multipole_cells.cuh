@@ -39,6 +39,16 @@ __device__ __forceinline__ double rsqrtNormal(double a)
     return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
+/// the arithmetic of root searches whose steps may move at the level of rounding
+struct NormalArithmetic {
+    static __device__ __forceinline__ double quotient(double a, double b)
+    {
+        const double y = rcpNormal(b), q = a * y;
+        return fma(fma(-b, q, a), y, q);
+    }
+    static __device__ __forceinline__ double root(double a) { return a > 1e-280 ? a * rsqrtNormal(a) : a >= 0 ? 0 : NAN; }
+};
+
 /// four consecutive doubles, 32-byte aligned, in one load: a lane's cell lies in lines of its own, and
 /// the L1's cost of a load is the number of different lines its lanes touch, so the width halves it
 __device__ __forceinline__ void ldg4(const double* p, double* v)
