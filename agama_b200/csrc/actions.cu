@@ -228,7 +228,7 @@ void runActions(const MultipoleView& M, const FudgeTables& F, long n, const doub
         mark(1);
         if(predict) bp->net->predict(count, feat, pred, stream);
         mark(2);
-        launchFudgeRoots(M, count, rec, ends, it, counter, pred, widths, bp ? bp->stats : nullptr, angles || !M.cells, stream);
+        launchFudgeRoots(M, count, rec, ends, it, counter, pred, widths, bp ? bp->stats : nullptr, angles, stream);
         mark(3);
         if(samples)
             launchBracketTargets(count, rec, samples->target + 3 * first, samples->mask + 3 * first, stream);

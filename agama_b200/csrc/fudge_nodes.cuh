@@ -111,6 +111,79 @@ __device__ __forceinline__ void limitRootEval(const FudgeFunction& f, int kind, 
     }
 }
 
+/// F(tau) of one branch (FudgeFunction::eval, to the bit) in a potential with cells, without calls;
+/// D2inv = 1 / D2
+static __device__ __forceinline__ double branchValue(const FudgeFunction& f, double D2inv, double tau)
+{
+    const MultipoleView& M = *f.M;
+    const bool lambda = tau >= f.D2;
+    const double lam = lambda ? tau : f.lambda, n = lambda ? fabs(f.nu) : tau;
+    const double mult = lambda ? lam - n : n - lam, I = lambda ? f.Ilam : f.Inu;
+    const double absnu = fabs(n), lmd = lam - f.D2, nmd = absnu - f.D2;
+    if(nmd > 0 || lmd < 0) return NAN;
+    // coordinates that leave the range of normal numbers take the library's roots
+    const double R2 = lmd * (1 - quotient(absnu, f.D2, D2inv)), z2 = quotient(lam * absnu, f.D2, D2inv);
+    const bool usual = R2 > 1e-200 && R2 < 1e200 && z2 > 1e-200 && z2 < 1e200;
+    const double R = usual ? squareRoot(R2) : sqrt(R2), z = (usual ? squareRoot(z2) : sqrt(z2)) * (n >= 0 ? 1 : -1);
+    const double rsq = sumProducts(z, z, R, R);
+    const double Phi = inCells(M, rsq) ? valueInterp2d(M, R, z) : axisPowerLaw<false>(rsq < M.rInnerSq ? M.inner : M.outer, R, z, rsq, nullptr, nullptr);
+    const double tmd = tau - f.D2;
+    return fma(-f.L2h, tau, tmd != 0 ? fma(-Phi, mult, fma(f.E, tau, -I)) * tmd : 0);
+}
+
+/// the same with F'(tau)
+static __device__ __forceinline__ void branchSlope(const FudgeFunction& f, double D2inv, double tau, double* val, double* der)
+{
+    const MultipoleView& M = *f.M;
+    const bool lambda = tau >= f.D2;
+    const double lam = lambda ? tau : f.lambda, n = lambda ? fabs(f.nu) : tau;
+    const double mult = lambda ? lam - n : n - lam, I = lambda ? f.Ilam : f.Inu;
+    const double absnu = fabs(n), lmd = lam - f.D2, nmd = absnu - f.D2;
+    if(nmd > 0 || lmd < 0) { *val = *der = NAN; return; }
+    const double R2 = lmd * (1 - quotient(absnu, f.D2, D2inv)), z2 = quotient(lam * absnu, f.D2, D2inv);
+    const bool usual = R2 > 1e-200 && R2 < 1e200 && z2 > 1e-200 && z2 < 1e200;
+    const double sgn = n >= 0 ? 1 : -1;
+    const double R = usual ? squareRoot(R2) : sqrt(R2), z = (usual ? squareRoot(z2) : sqrt(z2)) * sgn;
+    double Phi;
+    CylDerivs g;
+    const double rsq = sumProducts(R, R, z, z);     // (the value alone adds them the other way round)
+    if(inCells(M, rsq)) forceInterp2d<EVAL_AXI, 1, false>(M, R, z, rsq, 0, &Phi, &g);
+    else                Phi = axisPowerLaw<true>(rsq < M.rInnerSq ? M.inner : M.outer, R, z, rsq, &g.dR, &g.dz);
+    const double tmd = tau - f.D2;
+    *val = fma(-f.L2h, tau, tmd != 0 ? fma(-Phi, mult, fma(f.E, tau, -I)) * tmd : 0);
+    // dR/dtau, dz/dtau along the coordinate that tau moves
+    const double dR = lambda ? lmd : nmd, dz = lambda ? lam : n;
+    double dRdt, dzdt;
+    if(usual) { dRdt = quotient(0.5 * R, dR, reciprocal(dR)); dzdt = quotient(0.5 * z, dz, reciprocal(dz)); }
+    else      { dRdt = 0.5 * R / dR; dzdt = 0.5 * z / dz; }
+    if(!lambda) dRdt *= sgn;
+    const double dPhidtau = sumProducts(g.dR, dRdt, g.dz, dzdt);
+    *der = fma(-(mult + tmd), Phi, fma(f.E, tau + tmd, -f.L2h) - I) - (tmd != 0 ? tmd * mult * dPhidtau : 0);
+}
+
+/// limitRootEval of a potential with cells
+static __device__ __forceinline__ void limitRootSegments(const FudgeFunction& f, double D2inv, int kind, double u0, double x,
+    double* v, double* d)
+{
+    const bool semiInf = kind == ROOT_LAMBDA_MAX;
+    double duds = 1, tau = x;
+    if(semiInf) {       // unscaleSemiInf (u0 > Delta^2 > 0; x = 1 gives NaN: far)
+        const double w = 1 - x, w2 = pow2(w);
+        tau = u0 * exp(quotient(x, w, reciprocal(w)));
+        duds = quotient(tau, w2, reciprocal(w2));
+    }
+    const bool far = semiInf && !(tau <= 1e100);
+    double fval = 0, fder = 0;
+    if(!far) branchSlope(f, D2inv, tau, &fval, &fder);
+    if(!semiInf) { *v = fval; *d = fder; }
+    else if(far) { *v = f.E; *d = NAN; }
+    else {
+        const double tau2 = pow2(tau), y2 = reciprocal(tau2);
+        *v = quotient(fval, tau2, y2);
+        *d = quotient(fder - quotient(2 * fval, tau, reciprocal(tau)), tau2, y2) * duds;
+    }
+}
+
 /** Integration limits of the lambda and nu motions (findIntegrationLimitsAxisym,
     src/actions_staeckel.cpp:360-483), part 1: every decision up to the three root searches, whose
     brackets go into the record; limits that need no root are stored directly (NaN otherwise).
@@ -273,26 +346,6 @@ static __device__ AngleSetup fudgeAngleSetup(const MultipoleView& M, const Fudge
         a.yn = lim.nu_max == 0 ? 0 : scaleCubInverse(0, lim.nu_max, fabs(rec.nu));
     }
     return a;
-}
-
-/// F(tau) of one branch (FudgeFunction::eval, to the bit) in a potential with cells, without calls;
-/// D2inv = 1 / D2
-static __device__ __forceinline__ double branchValue(const FudgeFunction& f, double D2inv, double tau)
-{
-    const MultipoleView& M = *f.M;
-    const bool lambda = tau >= f.D2;
-    const double lam = lambda ? tau : f.lambda, n = lambda ? fabs(f.nu) : tau;
-    const double mult = lambda ? lam - n : n - lam, I = lambda ? f.Ilam : f.Inu;
-    const double absnu = fabs(n), lmd = lam - f.D2, nmd = absnu - f.D2;
-    if(nmd > 0 || lmd < 0) return NAN;
-    // coordinates that leave the range of normal numbers take the library's roots
-    const double R2 = lmd * (1 - quotient(absnu, f.D2, D2inv)), z2 = quotient(lam * absnu, f.D2, D2inv);
-    const bool usual = R2 > 1e-200 && R2 < 1e200 && z2 > 1e-200 && z2 < 1e200;
-    const double R = usual ? squareRoot(R2) : sqrt(R2), z = (usual ? squareRoot(z2) : sqrt(z2)) * (n >= 0 ? 1 : -1);
-    const double rsq = sumProducts(z, z, R, R);
-    const double Phi = inCells(M, rsq) ? valueInterp2d(M, R, z) : valuePowerLaw(rsq < M.rInnerSq ? M.inner : M.outer, R, z);
-    const double tmd = tau - f.D2;
-    return fma(-f.L2h, tau, tmd != 0 ? fma(-Phi, mult, fma(f.E, tau, -I)) * tmd : 0);
 }
 
 /// one node (abscissa x, weight w) of a branch integral over the scaled interval [0, y] of [lo, hi]

@@ -26,7 +26,7 @@ void launchNodePrepare(bool finder, const MultipoleView& M, const FudgeTables& F
 /// searches start on the predicted brackets; stats (4 counters, may be null) accumulates
 /// searches, narrowed searches, fallbacks to the plain bracket and iterations; ends (may be null):
 /// F and F' at the ends of each record's plain brackets, which the plain searches take instead of
-/// evaluating them again; nodes: F from the node form of the splines (records whose angles follow)
+/// evaluating them again; nodes: F to the bits of the node form of the splines (records whose angles follow)
 void launchFudgeRoots(const MultipoleView& M, long n, FudgeRecord* rec, const FudgeEnds* ends, int* iters,
     unsigned long long* counter, const float* pred, const BracketWidths& widths, unsigned long long* stats,
     bool nodes, cudaStream_t stream);

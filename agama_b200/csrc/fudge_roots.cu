@@ -28,6 +28,10 @@ __device__ __forceinline__ void storePlainLimit(FudgeRecord& r, int kind, const 
     else r.lambdaMax = unscaleSemiInf(u0, s.result, nullptr);
 }
 
+/// where F comes from: the cells (actions alone), the cells' segments (points whose angles follow: the bits
+/// of the node form) or the node form (potentials without cells)
+enum RootForm { ROOT_CELLS, ROOT_SEGMENTS, ROOT_NODES };
+
 /// what a lane does next with its search
 enum { LANE_IDLE = 0, LANE_PROPOSE = 1, LANE_EVAL = 2, LANE_VERIFY = 3 };
 
@@ -109,15 +113,15 @@ __device__ __forceinline__ bool predictedBracket(const FudgeRecord& r, int kind,
     be null) accumulates {searches, seeded searches, plain searches after a failed check,
     iterations} when STATS.  LEARNED = false (no predictions, no stats) compiles the plain searches
     alone, without that state and the counters (fewer registers); STATS = false leaves the
-    counters out of the learned searches.  NODES = true evaluates F from the node form of the splines
-    (points whose angles follow, potentials without cells), false from the cells: without a call in the
-    evaluation the searches fit 80 registers (1e6 disk points at 3 / 4 / 5 / 6 / 7 / 8 blocks per SM 1265 / 1015 /
-    930 / 908 / 945 / 1040 us; with the call and 370 B of spills 1150 at 4).  Quotients and roots of the
+    counters out of the learned searches.  FORM: where F comes from.  ROOT_CELLS: without a
+    call in the evaluation the searches fit 80 registers (1e6 disk points at 3 / 4 / 5 / 6 / 7 / 8 blocks per SM 1265 / 1015 /
+    930 / 908 / 945 / 1040 us; with the call and 370 B of spills 1150 at 4).  ROOT_SEGMENTS: the bits of the node form without
+    its calls and divisions (1e5 galaxy points 275 -> 207 us).  Quotients and roots of the
     searches' steps without the library's slow paths (NormalArithmetic): 919 -> 819 us, 366 B of spills; at 4 / 5 / 6 blocks
     869 / 812 / 805 us.  The learned searches hold more state: 4 blocks (2417 us a step with the counters, 2562 at 6).
     Bound by latency and issue together: 60 % of the issue slots, 19 of 32 lanes (the branches of a step). */
-template<bool LEARNED, bool STATS, bool NODES>
-__global__ void __launch_bounds__(ROOT_BLOCK, NODES || LEARNED ? 4 : 6) fudgeRootKernel(const __grid_constant__ MultipoleView M, long n,
+template<bool LEARNED, bool STATS, RootForm FORM>
+__global__ void __launch_bounds__(ROOT_BLOCK, FORM != ROOT_CELLS || LEARNED ? 4 : 6) fudgeRootKernel(const __grid_constant__ MultipoleView M, long n,
     FudgeRecord* __restrict__ rec, const FudgeEnds* __restrict__ ends, int* __restrict__ iters,
     unsigned long long* __restrict__ counter, const float* __restrict__ pred, const BracketWidths widths,
     unsigned long long* __restrict__ stats)
@@ -130,8 +134,10 @@ __global__ void __launch_bounds__(ROOT_BLOCK, NODES || LEARNED ? 4 : 6) fudgeRoo
     int kind = 0;
     double x = 0, u0 = 0, verified = 0;
     unsigned nSearch = 0, nSeeded = 0, nFallback = 0, nIter = 0;
-    std::conditional_t<NODES, FudgeFunction, FudgeBranch> fnc{};
-    RootSearchOf<std::conditional_t<NODES, ExactArithmetic, NormalArithmetic>> s;
+    std::conditional_t<FORM == ROOT_CELLS, FudgeBranch, FudgeFunction> fnc{};
+    double D2inv = 0;       // (ROOT_SEGMENTS)
+    RootSearchOf<std::conditional_t<FORM == ROOT_CELLS, NormalArithmetic,
+        std::conditional_t<FORM == ROOT_SEGMENTS, RoundedArithmetic, ExactArithmetic>>> s;
     // a plain search on the point's bracket again (after a seeded root failed its check)
     auto restartPlain = [&]() {
         const FudgeRecord& r = rec[point];
@@ -188,8 +194,9 @@ __global__ void __launch_bounds__(ROOT_BLOCK, NODES || LEARNED ? 4 : 6) fudgeRoo
                     if(r.roots & (1 << k)) {
                         point = i;
                         kind = 1 << k;
-                        if constexpr(NODES) loadFudgeFunction(M, r, fnc);
-                        else loadFudgeBranch(r, kind != ROOT_NU_MAX, fnc);
+                        if constexpr(FORM == ROOT_CELLS) loadFudgeBranch(r, kind != ROOT_NU_MAX, fnc);
+                        else loadFudgeFunction(M, r, fnc);
+                        if(FORM == ROOT_SEGMENTS) D2inv = reciprocal(r.D2);
                         u0 = r.lambdaPos;
                         const double lo = kind == ROOT_NU_MAX ? fabs(r.nu) : kind == ROOT_LAMBDA_MIN ? r.lambdaLower : 0;
                         const double hi = kind == ROOT_NU_MAX ? r.nuUpper : kind == ROOT_LAMBDA_MIN ? r.lambdaPos : 1;
@@ -243,7 +250,8 @@ __global__ void __launch_bounds__(ROOT_BLOCK, NODES || LEARNED ? 4 : 6) fudgeRoo
         // 3. F (and F') at the points of the lanes that have one
         double fx = 0, dx = 0;
         if(mode == LANE_EVAL || mode == LANE_VERIFY) {
-            if constexpr(NODES) limitRootEval(fnc, kind, u0, x, &fx, &dx);
+            if constexpr(FORM == ROOT_SEGMENTS) limitRootSegments(fnc, D2inv, kind, u0, x, &fx, &dx);
+            else if constexpr(FORM == ROOT_NODES) limitRootEval(fnc, kind, u0, x, &fx, &dx);
             else limitRootEval<true>(M, fnc, kind == ROOT_LAMBDA_MAX, u0, x, &fx, &dx);
         }
         // 4. the values fed to the searches
@@ -300,7 +308,7 @@ __global__ void bracketTargetKernel(long n, const FudgeRecord* __restrict__ rec,
 }
 
 /// resident blocks of a root-kernel variant on the current device (cached per device and variant)
-template<bool LEARNED, bool STATS, bool NODES>
+template<bool LEARNED, bool STATS, RootForm FORM>
 int rootGridSize()
 {
     static std::mutex mutex;
@@ -312,7 +320,7 @@ int rootGridSize()
     if(it != cache.end()) return it->second;
     int sms = 0, perSM = 0;
     AGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    AGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, fudgeRootKernel<LEARNED, STATS, NODES>, ROOT_BLOCK, 0));
+    AGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, fudgeRootKernel<LEARNED, STATS, FORM>, ROOT_BLOCK, 0));
     const int grid = std::max(1, sms * std::max(1, perSM));
     cache[dev] = grid;
     return grid;
@@ -321,14 +329,14 @@ int rootGridSize()
 }  // namespace
 
 namespace {
-template<bool LEARNED, bool STATS, bool NODES>
+template<bool LEARNED, bool STATS, RootForm FORM>
 void launchRoots(const MultipoleView& M, long n, FudgeRecord* rec, const FudgeEnds* ends, int* iters,
     unsigned long long* counter, const float* pred, const BracketWidths& widths, unsigned long long* stats,
     cudaStream_t stream)
 {
     const long tasks = (3 * n + ROOT_BLOCK - 1) / ROOT_BLOCK;
-    const long grid = std::min<long>(rootGridSize<LEARNED, STATS, NODES>(), tasks);
-    fudgeRootKernel<LEARNED, STATS, NODES><<<grid, ROOT_BLOCK, 0, stream>>>(M, n, rec, ends, iters, counter, pred, widths,
+    const long grid = std::min<long>(rootGridSize<LEARNED, STATS, FORM>(), tasks);
+    fudgeRootKernel<LEARNED, STATS, FORM><<<grid, ROOT_BLOCK, 0, stream>>>(M, n, rec, ends, iters, counter, pred, widths,
         stats);
     AGB_CUDA(cudaGetLastError());
 }
@@ -341,9 +349,13 @@ void launchFudgeRoots(const MultipoleView& M, long n, FudgeRecord* rec, const Fu
     if(n <= 0) return;
     AGB_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), stream));
     // learned or plain searches with the counters; predictions alone; plain searches
-    auto launch = stats ? (nodes ? launchRoots<true, true, true> : launchRoots<true, true, false>)
-                : pred  ? (nodes ? launchRoots<true, false, true> : launchRoots<true, false, false>)
-                        : (nodes ? launchRoots<false, false, true> : launchRoots<false, false, false>);
+    auto pick = [&](auto form) {
+        constexpr RootForm F = decltype(form)::value;
+        return stats ? launchRoots<true, true, F> : pred ? launchRoots<true, false, F> : launchRoots<false, false, F>;
+    };
+    auto launch = !M.cells ? pick(std::integral_constant<RootForm, ROOT_NODES>())
+                : nodes    ? pick(std::integral_constant<RootForm, ROOT_SEGMENTS>())
+                           : pick(std::integral_constant<RootForm, ROOT_CELLS>());
     launch(M, n, rec, ends, iters, counter, pred, widths, stats, stream);
 }
 

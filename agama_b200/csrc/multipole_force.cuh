@@ -40,6 +40,14 @@ __device__ __forceinline__ double squareRoot(double a)
     return fma(fma(-g, g, a), 0.5 * y, g);
 }
 
+/// the divisions and roots of the root searches, correctly rounded without the library's slow paths (for operands
+/// outside the range of normal numbers a quotient is NaN where the library gives 0, NaN or an infinity: the
+/// searches refuse such steps alike)
+struct RoundedArithmetic {
+    static __device__ __forceinline__ double quotient(double a, double b) { return agb::quotient(a, b, reciprocal(b)); }
+    static __device__ __forceinline__ double root(double a) { return a > 1e-280 ? squareRoot(a) : sqrt(a); }
+};
+
 /// the basis of a quintic segment at one point (quinticSegmentR): f = fl + bf d0 + dx f1l + b1 d1 + e f2l + b2 d2,
 /// f' = bfp d0 + f1l + b1p d1 + dx f2l + b2p d2
 struct SegmentBasis {
@@ -130,14 +138,14 @@ __device__ __forceinline__ void segmentCell(const double* __restrict__ c, const 
     falls), so nothing is kept per harmonic.
     G > 1: the lanes of a group take G harmonics at a time, one each, and every lane adds all of them
     in the same order from the lane that evaluated it, so every G gives the same bits.
-    MIXED: the m != 0 harmonics from the FP32 table. */
+    MIXED: the m != 0 harmonics from the FP32 table.  rsq: R^2 + z^2, rounded as the caller wants it. */
 template<int KIND, int G, bool MIXED>
-__device__ __forceinline__ void forceInterp2d(const MultipoleView& M, double R, double z, double phi, double* pot,
+__device__ __forceinline__ void forceInterp2d(const MultipoleView& M, double R, double z, double rsq, double phi, double* pot,
     CylDerivs* g)
 {
     const int gl = G > 1 ? static_cast<int>(threadIdx.x % G) : 0;
     const unsigned gmask = G > 1 ? groupMask<G>() : 0u;
-    const double r = squareRoot(sumProducts(z, z, R, R)), logr = log(r), rpRinv = reciprocal(r + fabs(R));
+    const double r = squareRoot(rsq), logr = log(r), rpRinv = reciprocal(r + fabs(R));
     const double tau = R == 0 ? signOf(z) : z * rpRinv;
     const bool inside = logr >= M.gridR.x0 && logr <= M.gridR.xEnd && tau >= M.gridTau.x0 && tau <= M.gridTau.xEnd;
     double xl, xh, yl, yh, xhi, yhi;
@@ -368,15 +376,17 @@ __device__ __forceinline__ double valueInterp2d(const MultipoleView& M, double R
     return P;
 }
 
-/// the potential alone of an axisymmetric asymptotic expansion (evalPowerLaw): one short loop, inline
-__device__ __forceinline__ double valuePowerLaw(const PowerLawView& A, double R, double z)
+/// an axisymmetric asymptotic expansion (evalPowerLaw), with SLOPE its gradient over R and z: one short
+/// loop, inline; rsq: R^2 + z^2, rounded as the caller wants it
+template<bool SLOPE>
+__device__ __forceinline__ double axisPowerLaw(const PowerLawView& A, double R, double z, double rsq, double* gR, double* gz)
 {
     const HarmIndices& ind = A.ind;
-    const double rsq = sumProducts(z, z, R, R), dlogr = log(rsq / A.r0sq) * 0.5;
+    const double dlogr = log(rsq / A.r0sq) * 0.5;
     const int lmax = (A.inner && rsq < A.r0sq * 1e-16) || (!A.inner && rsq > A.r0sq * 1e16) ? 0 : ind.lmax;
     const double tau = z == 0 ? 0 : z / (sqrt(rsq) + R);
-    const double ct = 2 * tau / (1 + tau * tau);
-    double prefact = PMM_NORM_DEV[0], sum = 0, Plm1 = 1, Plm = 1, Plm2 = 0;
+    const double ct = 2 * tau / (1 + tau * tau), st = SLOPE ? (1 - tau * tau) / (1 + tau * tau) : 0, stInv = SLOPE ? 1 / st : 0;
+    double prefact = PMM_NORM_DEV[0], sum = 0, sumr = 0, sumt = 0, Plm1 = 1, Plm = 1, Plm2 = 0;
     for(int l = 0; l <= lmax; l++) {
         if(l == 1) Plm = ct * Plm1;
         else if(l > 1) {
@@ -389,13 +399,36 @@ __device__ __forceinline__ double valuePowerLaw(const PowerLawView& A, double R,
             const double s = ldg(A.S + c), u = ldg(A.U + c), w = ldg(A.W + c), v = A.inner ? l : -l - 1;
             const double rv = v != 0 ? exp(dlogr * v) : 1;
             const double rs = s != v ? (s != 0 && u != 0 ? exp(dlogr * s) : 1) : rv;
-            const double urs = u * rs * (s != v || u == 0 ? 1 : dlogr);
-            const double C = __dadd_rn(urs, w * rv) + (v == 0 ? A.Q * rsq / A.r0sq : 0);
-            if(lmax == 0) return C;
-            sum = fma(Plm * prefact * C, 2 * SQRT_PI, sum);
+            const double urs = u * rs * (s != v || u == 0 ? 1 : dlogr), wrv = w * rv;
+            const double qr2 = v == 0 ? A.Q * rsq / A.r0sq : 0;
+            const double C = __dadd_rn(urs, wrv) + qr2;
+            double dC = 0;
+            if(SLOPE) dC = sumProducts(wrv, v, urs, s) + (s != v ? 0 : u * rs) + qr2 * 2;
+            if(lmax == 0) {
+                if(SLOPE) {
+                    const double rsqinv = rsq > 0 ? 1 / rsq : 0;
+                    *gR = dC * (rsq < INFINITY ? R * rsqinv : 0);
+                    *gz = dC * (rsq < INFINITY ? z * rsqinv : 0);
+                }
+                return C;
+            }
+            const double P = Plm * prefact;
+            sum = fma(P * C, 2 * SQRT_PI, sum);
+            if(SLOPE) {
+                sumr = fma(P * dC, 2 * SQRT_PI, sumr);
+                const double dPlm = l == 0 ? 0 :
+                    st >= 1e-8 ? quotient(sumProducts(l * ct, Plm, -l, Plm1), st, stInv) :
+                    -l * (l + 1) / 2 * st * (ct > 0 || l % 2 == 1 ? 1 : -1);
+                sumt = fma(prefact * dPlm * C, 2 * SQRT_PI, sumt);
+            }
         }
         Plm2 = Plm1;
         Plm1 = Plm;
+    }
+    if(SLOPE) {
+        const double r2inv = 1 / rsq, drdR = R * r2inv, drdz = z * r2inv;
+        *gR = sumProducts(sumr, drdR, sumt, drdz);
+        *gz = sumProducts(sumr, drdz, sumt, -drdR);
     }
     return sum;
 }
@@ -449,7 +482,7 @@ __device__ __forceinline__ void evalForceCar(const MultipoleView& M, double x, d
         CylHess h;
         evalMultipoleCyl<3, KIND>(M, R, z, phi, pot, &g, &h);
     } else if(inCells(M, rsq))
-        forceInterp2d<KIND, G, MIXED>(M, R, z, phi, pot, &g);
+        forceInterp2d<KIND, G, MIXED>(M, R, z, sumProducts(z, z, R, R), phi, pot, &g);
     else {      // (results of this branch's own: the common ones stay in registers)
         double p;
         CylDerivs d;
