@@ -162,7 +162,9 @@ struct FudgeBranch {
         const double n = fabs(nu), lmd = lambda - D2, inv = rcpNormal(D2);
         mo = lam ? n : lambda;
         ro = lam ? n : lmd;
-        c1 = NormalArithmetic::root(lam ? 1 - n * inv : lmd * inv);
+        // D2 - n is exact near the axis and 0 on it (|z| > Delta), where 1 - n * inv is the rounding of the
+        // reciprocal, of either sign
+        c1 = NormalArithmetic::root((lam ? fmax(D2 - n, 0.) : lmd) * inv);
         c2 = NormalArithmetic::root((lam ? n : lambda) * inv);
     }
 
