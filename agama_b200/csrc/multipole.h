@@ -52,7 +52,7 @@ struct PowerLawView {
 struct alignas(16) GridNode { double x, invH; };
 struct GridView {
     const GridNode* cell;
-    const unsigned short* lut;
+    const int* lut;
     double x0, xEnd, lutScale;      // first and last node, nlut / (xEnd - x0)
     int n, nlut;
 };

@@ -251,7 +251,7 @@ DevicePotential* createDevicePotential(const std::vector<double>& radii,
         }
         for(int s = V.nFast; s < FAST_MAX_HARMONICS; s++) { V.fastM[s] = 0; V.fastSlot[s] = 0; }
         if(H.is2d) {
-            auto gridView = [](const std::vector<double>& g, DevBuf<GridNode>& cell, DevBuf<unsigned short>& lut) {
+            auto gridView = [](const std::vector<double>& g, DevBuf<GridNode>& cell, DevBuf<int>& lut) {
                 const int n = static_cast<int>(g.size());
                 std::vector<GridNode> c(n);
                 double narrowest = INFINITY;
@@ -269,11 +269,11 @@ DevicePotential* createDevicePotential(const std::vector<double>& radii,
                 v.lutScale = v.nlut / (v.xEnd - v.x0);
                 // the edge is moved down by a millionth of a bin: a value just below it may be put
                 // into this bin by the rounding of (x - x0) * lutScale
-                std::vector<unsigned short> l(v.nlut);
+                std::vector<int> l(v.nlut);
                 for(int b = 0, k = 0; b < v.nlut; b++) {
                     const double edge = v.x0 + (b - 1e-6) / v.lutScale;
                     while(k < n - 2 && g[k + 1] <= edge) k++;
-                    l[b] = static_cast<unsigned short>(k);
+                    l[b] = k;
                 }
                 cell.upload(c);
                 lut.upload(l);
@@ -281,8 +281,8 @@ DevicePotential* createDevicePotential(const std::vector<double>& radii,
                 v.lut = lut.ptr;
                 return v;
             };
-            if(H.lnr.size() < 2 || H.tau.size() < 2 || H.lnr.size() > 65535 || H.tau.size() > 65535)
-                throw std::invalid_argument("Multipole: the grids need between 2 and 65535 nodes");
+            if(H.lnr.size() < 2 || H.tau.size() < 2)
+                throw std::invalid_argument("Multipole: the grids need at least 2 nodes");
             V.gridR = gridView(H.lnr, P->gridCellR, P->gridLutR);
             V.gridTau = gridView(H.tau, P->gridCellTau, P->gridLutTau);
             // squares of radii outside the range of normal numbers stay with the node form

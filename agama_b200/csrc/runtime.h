@@ -49,7 +49,7 @@ struct DevicePotential {
     DevBuf<double> lnr, tau, lnrInvH, tauInvH, spl2d, spl1d, innerS, innerU, innerW, outerS, outerU, outerW;
     DevBuf<GridNode> gridCellR, gridCellTau;
     DevBuf<double> cells, segments, legendreNorm;
-    DevBuf<unsigned short> gridLutR, gridLutTau;
+    DevBuf<int> gridLutR, gridLutTau;
     DevBuf<float> spl2d32;
     MultipoleView view;
     /// the axisymmetric (m = 0) part, used by the action finder (same as the full potential
