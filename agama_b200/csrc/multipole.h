@@ -9,7 +9,7 @@
 #include <vector>
 #include <string>
 #include <map>
-#include "common.cuh"
+#include "grid_cells.h"
 
 namespace agb {
 
@@ -42,21 +42,6 @@ struct PowerLawView {
     const double* W;      // amplitudes of (r/r0)^v
     const double* norm;   // [m][l]: sqrt((2l+1)/(2l-1) (l-m)/(l+m)), stride LMAX_MAX + 1
 };
-
-/** device view of one grid of the 2-D splines, for the search of the cell that holds a value: cell
-    k < n - 1 is (node k, 1 / (node k+1 - node k)) and entry n - 1 the last node, so that two
-    neighbouring 16-byte loads give both nodes of a cell and its reciprocal width.  lut[b] is the
-    last cell that begins at or before the left edge of bin b of an even division of the grid into
-    nlut bins; the bins are at most half as wide as the narrowest cell (up to GRID_LUT_MAX of them),
-    so the search almost never goes beyond the next cell. */
-struct alignas(16) GridNode { double x, invH; };
-struct GridView {
-    const GridNode* cell;
-    const int* lut;
-    double x0, xEnd, lutScale;      // first and last node, nlut / (xEnd - x0)
-    int n, nlut;
-};
-constexpr int GRID_LUT_MAX = 4096;
 
 /// number of coefficients of one cell of a 2-D spline in monomial form
 constexpr int CELL_COEFS = 36;

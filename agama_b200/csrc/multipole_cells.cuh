@@ -56,19 +56,13 @@ __device__ __forceinline__ void ldg4(const double* p, double* v)
     asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3]) : "l"(p));
 }
 
-/// the cell of a grid that holds x (x0 <= x <= xEnd; the last node belongs to the last cell): its
-/// index, nodes and reciprocal width.  For x outside or NaN the result is some cell of the grid.
+/// findCell from device tables: index, nodes and reciprocal width of the cell
 __device__ __forceinline__ int gridCell(const GridView& g, double x, double* xl, double* xh, double* invH)
 {
-    const int b = min(max(__double2int_rz((x - g.x0) * g.lutScale), 0), g.nlut - 1);
-    int k = __ldg(g.lut + b);
-    double2 lo = ldg2(&g.cell[k].x), hi = ldg2(&g.cell[k + 1].x);
-    while(x >= hi.x && k < g.n - 2) {
-        k++;
-        lo = hi;
-        hi = ldg2(&g.cell[k + 1].x);
-    }
-    *xl = lo.x; *xh = hi.x; *invH = lo.y;
+    GridNode lo, hi;
+    const int k = findCell(g, x, &lo, &hi, [&](int i) { const double2 v = ldg2(&g.cell[i].x); return GridNode{ v.x, v.y }; },
+        [&](int b) { return __ldg(g.lut + b); });
+    *xl = lo.x; *xh = hi.x; *invH = lo.invH;
     return k;
 }
 

@@ -1,7 +1,6 @@
 // Multipole potential on the device: table upload and the batched evaluation kernel.
 #include "runtime.h"
 #include "multipole_cells.cuh"
-#include <algorithm>
 
 namespace agb {
 
@@ -252,29 +251,10 @@ DevicePotential* createDevicePotential(const std::vector<double>& radii,
         for(int s = V.nFast; s < FAST_MAX_HARMONICS; s++) { V.fastM[s] = 0; V.fastSlot[s] = 0; }
         if(H.is2d) {
             auto gridView = [](const std::vector<double>& g, DevBuf<GridNode>& cell, DevBuf<int>& lut) {
-                const int n = static_cast<int>(g.size());
-                std::vector<GridNode> c(n);
-                double narrowest = INFINITY;
-                for(int k = 0; k < n; k++) {
-                    c[k].x = g[k];
-                    c[k].invH = k + 1 < n ? 1 / (g[k + 1] - g[k]) : 0;
-                    if(k + 1 < n) narrowest = std::min(narrowest, g[k + 1] - g[k]);
-                }
+                std::vector<GridNode> c;
+                std::vector<int> l;
                 GridView v;
-                v.n = n;
-                v.x0 = g.front();
-                v.xEnd = g.back();
-                const double bins = 2 * (v.xEnd - v.x0) / narrowest;
-                v.nlut = bins < GRID_LUT_MAX ? std::max(1, static_cast<int>(bins) + 1) : GRID_LUT_MAX;
-                v.lutScale = v.nlut / (v.xEnd - v.x0);
-                // the edge is moved down by a millionth of a bin: a value just below it may be put
-                // into this bin by the rounding of (x - x0) * lutScale
-                std::vector<int> l(v.nlut);
-                for(int b = 0, k = 0; b < v.nlut; b++) {
-                    const double edge = v.x0 + (b - 1e-6) / v.lutScale;
-                    while(k < n - 2 && g[k + 1] <= edge) k++;
-                    l[b] = k;
-                }
+                makeGridTables(g, &c, &l, &v);
                 cell.upload(c);
                 lut.upload(l);
                 v.cell = cell.ptr;
