@@ -289,7 +289,8 @@ __device__ __forceinline__ bool evalCellsCar(const MultipoleView& M, double x, d
         double d2Rdx2 = 1, d2Rdy2 = 1, d2Rdxdy = 1, d2phidx2 = 1, d2phidy2 = 1, d2phidxdy = 1;
         if(!axis) {
             d2Rdx2 = s * s * Rinv; d2Rdy2 = c * c * Rinv; d2Rdxdy = -s * c * Rinv;
-            d2phidx2 = 2 * s * c * (Rinv * Rinv); d2phidy2 = -d2phidx2; d2phidxdy = (s * s - c * c) * (Rinv * Rinv);
+            // (factor by factor: the square of 1 / R overflows where the factor before it can be 0)
+            d2phidx2 = 2 * s * c * Rinv * Rinv; d2phidy2 = -d2phidx2; d2phidxdy = (s * s - c * c) * Rinv * Rinv;
         }
         hess[0] = (h.dR2 * dRdx + h.dRdphi * dphidx) * dRdx + (h.dRdphi * dRdx + h.dphi2 * dphidx) * dphidx +
                   g.dR * d2Rdx2 + g.dphi * d2phidx2;                                         // xx
