@@ -257,12 +257,13 @@ __device__ __forceinline__ void evalCellsCyl(const MultipoleView& M, double R, d
     }
 }
 
-/// a Cartesian point beyond the cells (or of a potential without them), out of line
-template<int NQ>
+/// a Cartesian point beyond the cells (or of a potential without them), out of line; for an axisymmetric
+/// potential without the azimuth, whose derivatives are NaN at infinite points
+template<int NQ, int KIND>
 __device__ __noinline__ void evalBeyondCellsCar(const MultipoleView& M, double x, double y, double z, double* pot,
     double* grad, double* hess)
 {
-    evalMultipoleCar<NQ, EVAL_GENERAL>(M, x, y, z, pot, grad, hess);
+    evalMultipoleCar<NQ, KIND>(M, x, y, z, pot, grad, hess);
 }
 
 /** Evaluation at a Cartesian point with gradient (and Hessian xx,yy,zz,xy,yz,zx) in Cartesian

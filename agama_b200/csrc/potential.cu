@@ -37,7 +37,7 @@ __global__ void __launch_bounds__(128, NQ == 6 ? 4 : 6) evalPotentialKernel(cons
         }
     }
     double p, g[3], h[6];       // (variables of the rare path's own: its call takes their addresses)
-    evalBeyondCellsCar<NQ>(M, x, y, z, &p, g, h);
+    evalBeyondCellsCar<NQ, KIND>(M, x, y, z, &p, g, h);
     store(p, g, h);
 }
 
