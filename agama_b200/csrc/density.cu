@@ -106,7 +106,7 @@ __device__ __noinline__ double axisDensity(const MultipoleView& M, double R, dou
 
 /// the rare interiors without cells (lmax <= 2, many harmonics) away from the axis
 template<int KIND>
-__device__ __noinline__ double nodeDensity(const MultipoleView& M, double R, double z, double phi)
+__device__ __forceinline__ double nodeDensity(const MultipoleView& M, double R, double z, double phi)
 {
     CylDerivs g; CylHess h;
     interiorDerivs<KIND>(M, R, z, phi, &g, &h);

@@ -248,22 +248,14 @@ __device__ __forceinline__ void evalCellsCyl(const MultipoleView& M, double R, d
         double sphi = 0, cphi = 1;
         if(KIND == EVAL_FAST) sincos(phi, &sphi, &cphi);
         evalCells<NQ, KIND>(M, R, z, cphi, sphi, pot, g, h);
-    } else {
-        BeyondCells r;
-        evalBeyondCells<NQ>(M, R, z, phi, &r);
-        *pot = r.pot;
-        if(NQ >= 3) *g = r.g;
-        if(NQ == 6) *h = r.h;
+    } else {        // (a result of this branch's own, whose address the calls in it take)
+        double p;
+        CylDerivs d; CylHess dd;
+        evalMultipoleCyl<NQ, KIND>(M, R, z, phi, &p, &d, &dd);
+        *pot = p;
+        if(NQ >= 3) *g = d;
+        if(NQ == 6) *h = dd;
     }
-}
-
-/// a Cartesian point beyond the cells (or of a potential without them), out of line; for an axisymmetric
-/// potential without the azimuth, whose derivatives are NaN at infinite points
-template<int NQ, int KIND>
-__device__ __noinline__ void evalBeyondCellsCar(const MultipoleView& M, double x, double y, double z, double* pot,
-    double* grad, double* hess)
-{
-    evalMultipoleCar<NQ, KIND>(M, x, y, z, pot, grad, hess);
 }
 
 /** Evaluation at a Cartesian point with gradient (and Hessian xx,yy,zz,xy,yz,zx) in Cartesian

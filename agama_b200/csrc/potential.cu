@@ -7,15 +7,24 @@ namespace agb {
 namespace {
 thread_local std::string g_error;
 
+/// Blocks of 128 per SM that the registers are cut for: points beyond the radial grid wait for the
+/// logarithms and powers of the expansions, and the cells for their loads, so more warps are worth some
+/// spilled registers.  Potential alone at 6 / 8 blocks: 54.0 / 51.5 us inside the grid, 99 / 88 beyond it (1e6 points,
+/// disk potential); value and gradient at 5 / 6: 58.0 / 56.0, 123 / 115; with the Hessian at 3 / 4: 76 / 73, 236 / 199.
+/// Potentials without cells keep the compiler's own choice (96 to 228 registers; 1e6 points of one with 17
+/// harmonics: 436 us, 461 at 6 blocks, 517 at one).
+constexpr int minBlocks(int nq, int kind) { return kind == EVAL_GENERAL ? 0 : nq == 1 ? 8 : nq == 3 ? 6 : 4; }
+
 /// One point per thread; 128 threads per block.  NQ = 1 (potential), 3 (+gradient), 6 (+Hessian);
 /// KIND = spline evaluator matching the potential (EvalKind).  Bound by the L1: each lane reads its own
 /// cells, nine 32-byte loads a harmonic at one data-stage cycle per lane (60 % of its rate at 2e6
 /// points of the triaxial lmax 6 potential, value and gradient: 543 us from the node form at 168
 /// registers, 410 from the cells with 16-byte loads at 80 registers, 330 with 32-byte loads, 305 with the
-/// sign applied here instead of in a pass of its own; with the Hessian and the density at 4e5 points 294 -> 174 -> 163 us).
+/// sign applied here instead of in a pass of its own, 298 with the expansions inline; Hessian and density of 4e5
+/// points of the bar potential: 295 -> 161 us).
 /// gradSign, hessSign: 1, or -1 for the acceleration and its derivatives.
 template<int NQ, int KIND>
-__global__ void __launch_bounds__(128, NQ == 6 ? 4 : 6) evalPotentialKernel(const __grid_constant__ MultipoleView M, long n,
+__global__ void __launch_bounds__(128, minBlocks(NQ, KIND)) evalPotentialKernel(const __grid_constant__ MultipoleView M, long n,
     const double* __restrict__ pos, double* __restrict__ phi, double* __restrict__ grad,
     double* __restrict__ hess, double gradSign, double hessSign)
 {
@@ -29,15 +38,15 @@ __global__ void __launch_bounds__(128, NQ == 6 ? 4 : 6) evalPotentialKernel(cons
         if(NQ == 6 && hess)
             for(int k = 0; k < 6; k++) hess[6 * i + k] = hessSign * h[k];
     };
-    if(KIND != EVAL_GENERAL) {
-        double p, g[3], h[6];
-        if(evalCellsCar<NQ, KIND == EVAL_GENERAL ? EVAL_AXI : KIND>(M, x, y, z, &p, g, h)) {
-            store(p, g, h);
-            return;
-        }
+    double p, g[3], h[6];
+    if constexpr(KIND == EVAL_GENERAL)
+        evalMultipoleCar<NQ, KIND>(M, x, y, z, &p, g, h);
+    else if(!evalCellsCar<NQ, KIND>(M, x, y, z, &p, g, h)) {
+        double pb, gb[3], hb[6];    // (variables of the rare path's own, whose calls take their addresses)
+        evalMultipoleCar<NQ, KIND>(M, x, y, z, &pb, gb, hb);
+        store(pb, gb, hb);
+        return;
     }
-    double p, g[3], h[6];       // (variables of the rare path's own: its call takes their addresses)
-    evalBeyondCellsCar<NQ, KIND>(M, x, y, z, &p, g, h);
     store(p, g, h);
 }
 
@@ -46,7 +55,7 @@ __global__ void __launch_bounds__(128, NQ == 6 ? 4 : 6) evalPotentialKernel(cons
 /// reference's BasePotentialCyl::evalCyl returns them (no round trip through Cartesian
 /// derivatives, which loses the phi derivatives to cancellation at large R)
 template<int NQ, int KIND>
-__global__ void __launch_bounds__(128, NQ == 6 ? 4 : 6) evalPotentialCylKernel(const __grid_constant__ MultipoleView M, long n,
+__global__ void __launch_bounds__(128, minBlocks(NQ, KIND)) evalPotentialCylKernel(const __grid_constant__ MultipoleView M, long n,
     const double* __restrict__ pos, double* __restrict__ phi, double* __restrict__ grad,
     double* __restrict__ hess)
 {
