@@ -25,7 +25,9 @@ __device__ __forceinline__ double quotient(double a, double b, double y)
     return fma(fma(-b, q1, a), y, q1);
 }
 
-/// 1 / b correctly rounded, for b well inside the range of normal numbers (the same step)
+/// 1 / b correctly rounded, for b well inside the range of normal numbers (the same step); the one exception
+/// is a b whose fraction is of ones alone, left a unit low where the approximation is (Markstein's; its
+/// quotients are right all the same)
 __device__ __forceinline__ double reciprocal(double b)
 {
     const double y = rcpNormal(b);
@@ -377,7 +379,9 @@ __device__ __forceinline__ double valueInterp2d(const MultipoleView& M, double R
 }
 
 /// an axisymmetric asymptotic expansion (evalPowerLaw), with SLOPE its gradient over R and z: one short
-/// loop, inline; rsq: R^2 + z^2, rounded as the caller wants it
+/// loop, inline; rsq: R^2 + z^2, rounded as the caller wants it.  The same sums, but not to the bit:
+/// the contractions of evalPowerLaw are the compiler's, and expansions of lmax 2 take the recurrence
+/// here and a closed form there.
 template<bool SLOPE>
 __device__ __forceinline__ double axisPowerLaw(const PowerLawView& A, double R, double z, double rsq, double* gR, double* gz)
 {
