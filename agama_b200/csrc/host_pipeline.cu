@@ -6,10 +6,10 @@
 #include <chrono>
 #include <cstdint>
 #include <cstring>
+#include <exception>
 #include <map>
 #include <memory>
 #include <mutex>
-#include <system_error>
 #include <thread>
 
 namespace agb {
@@ -102,7 +102,7 @@ public:
         threads_.reserve(count);
         try {
             for(size_t t = 0; t < count; t++) threads_.emplace_back([this] { work(); });
-        } catch(const std::system_error&) {}    // a thread could not be started: the ones that run do the work
+        } catch(const std::exception&) {}       // no thread or no memory for one more: the ones that run do the work
     }
     bool running() const { return !threads_.empty(); }
     ~Stager()
