@@ -24,7 +24,11 @@ constexpr size_t ALIGN = 256;
 /// staging of pageable inputs: pieces of a megabyte through a ring of page-locked memory
 constexpr size_t PIECE = 1 << 20;
 constexpr int RING = 16, STAGING_THREADS = 4;
-constexpr size_t MIN_STAGED = 4 * PIECE;        // smaller inputs are copied as they are
+/// smaller inputs are copied as they are: starting the threads and handing over the pieces costs ~0.4 ms,
+/// which the faster copies earn back from here on (copied / staged at 4, 16, 24, 28, 48 MB: potentials
+/// 0.36 / 0.85, 1.00 / 1.15, 1.41 / 1.33, 1.65 / 1.52, 4.0 / 2.1 ms; actions 0.53 / 0.96, 1.30 / 1.64,
+/// 1.81 / 1.70, 2.12 / 1.88, 3.7 / 2.6 ms)
+constexpr size_t MIN_STAGED = 28 * PIECE;
 constexpr size_t MAX_IDLE_RINGS = 4;            // rings kept by stream sets that are not in use
 
 /// a set of non-blocking streams of one device, with its staging ring (allocated when first needed),
