@@ -17,10 +17,9 @@ namespace agb {
 /// the fudge's auxiliary function F(tau) and the integrals of motion of one point
 struct FudgeFunction {
     const MultipoleView* M;
-    double lambda, nu, phi, D2;     // point in prolate spheroidal coordinates (Delta^2 = D2)
+    double lambda, nu, D2;          // point in prolate spheroidal coordinates (Delta^2 = D2)
     double E, Lz, I3, flambda, fnu;
     double Ilam, Inu, L2h;          // I3 - fnu, I3 - flambda and Lz^2 / 2, formed once (derive())
-    int bad;                        // set when a coordinate conversion is invalid
 
     /// the terms of F that do not depend on tau, from the integrals of motion (the same
     /// operations as in F itself, so the same bits)
@@ -45,10 +44,10 @@ struct FudgeFunction {
         const double z = sqrt(lam * absnu / D2) * sgn;
         double Phi;
         CylDerivs g; CylHess h;
-        if(INL)      evalMultipoleCyl<DER2 ? 6 : DER ? 3 : 1, EVAL_AXI>(*M, R, z, phi, &Phi, &g, &h);
-        else if(DER2) evalMultipoleCylCall<6, EVAL_AXI>(*M, R, z, phi, &Phi, &g, &h);
-        else if(DER) evalMultipoleCylCall<3, EVAL_AXI>(*M, R, z, phi, &Phi, &g, &h);
-        else         evalMultipoleCylCall<1, EVAL_AXI>(*M, R, z, phi, &Phi, &g, &h);
+        if(INL)      evalMultipoleCyl<DER2 ? 6 : DER ? 3 : 1, EVAL_AXI>(*M, R, z, 0, &Phi, &g, &h);
+        else if(DER2) evalMultipoleCylCall<6, EVAL_AXI>(*M, R, z, 0, &Phi, &g, &h);
+        else if(DER) evalMultipoleCylCall<3, EVAL_AXI>(*M, R, z, 0, &Phi, &g, &h);
+        else         evalMultipoleCylCall<1, EVAL_AXI>(*M, R, z, 0, &Phi, &g, &h);
         const double tmd = tau - D2;
         *val = (tmd != 0 ? (E * tau - I - Phi * mult) * tmd : 0) - L2h * tau;
         if(DER || DER2) {
@@ -87,10 +86,9 @@ struct FudgeFunction {
 __device__ __forceinline__ void loadFudgeFunction(const MultipoleView& M, const FudgeRecord& r, FudgeFunction& f)
 {
     f.M = &M;
-    f.lambda = r.lambda; f.nu = r.nu; f.phi = 0; f.D2 = r.D2;
+    f.lambda = r.lambda; f.nu = r.nu; f.D2 = r.D2;
     f.E = r.E; f.Lz = r.Lz; f.I3 = r.I3; f.flambda = r.flambda; f.fnu = r.fnu;
     f.derive();
-    f.bad = 0;
 }
 
 /// the root functions of the integration limits (as limitRootEval of the cells' form)
@@ -187,10 +185,10 @@ static __device__ __forceinline__ void limitRootSegments(const FudgeFunction& f,
 /** Integration limits of the lambda and nu motions (findIntegrationLimitsAxisym,
     src/actions_staeckel.cpp:360-483), part 1: every decision up to the three root searches, whose
     brackets go into the record; limits that need no root are stored directly (NaN otherwise).
-    ends (may be null) receives F and F' at the ends of the plain brackets (FudgeEnds), which the
+    ends receives F and F' at the ends of the plain brackets (FudgeEnds), which the
     root searches then take instead of evaluating them: at lambda_pos from the evaluation above,
     at Delta^2 and |nu| from the same evaluation of F as the searches would make. */
-static __device__ void nodeLimitsSetup(const FudgeFunction& fnc, FudgeRecord& rec, FudgeEnds* ends = nullptr)
+static __device__ void nodeLimitsSetup(const FudgeFunction& fnc, FudgeRecord& rec, FudgeEnds* ends)
 {
     const double delta = fnc.D2;
     const double f_zero = fnc.value(0);
@@ -238,14 +236,12 @@ static __device__ void nodeLimitsSetup(const FudgeFunction& fnc, FudgeRecord& re
     rec.nuMax = nu_max; rec.lambdaMin = lambda_min; rec.lambdaMax = lambda_max;
     rec.nuUpper = nu_upper; rec.lambdaLower = lambda_lower; rec.lambdaPos = lambda_pos;
     rec.roots = roots;
-    if(ends) {
-        ends->fPos = f_pos; ends->dfPos = df_pos;
-        ends->fD2 = ends->dfD2 = ends->fNu = ends->dfNu = NAN;
-        if(((roots & ROOT_NU_MAX) && nu_upper == delta) || ((roots & ROOT_LAMBDA_MIN) && lambda_lower == delta))
-            fnc.eval<true, false>(delta, &ends->fD2, &ends->dfD2, nullptr);
-        if(roots & ROOT_NU_MAX)
-            fnc.eval<true, false>(fabs(fnc.nu), &ends->fNu, &ends->dfNu, nullptr);
-    }
+    ends->fPos = f_pos; ends->dfPos = df_pos;
+    ends->fD2 = ends->dfD2 = ends->fNu = ends->dfNu = NAN;
+    if(((roots & ROOT_NU_MAX) && nu_upper == delta) || ((roots & ROOT_LAMBDA_MIN) && lambda_lower == delta))
+        fnc.eval<true, false>(delta, &ends->fD2, &ends->dfD2, nullptr);
+    if(roots & ROOT_NU_MAX)
+        fnc.eval<true, false>(fabs(fnc.nu), &ends->fNu, &ends->dfNu, nullptr);
 }
 
 /** Phase 1 of the actions of one point (R, z, phi, vR, vz, vphi) for focal distance fd
@@ -255,7 +251,7 @@ static __device__ void nodeLimitsSetup(const FudgeFunction& fnc, FudgeRecord& re
     Otherwise the record holds the integrals of motion (findIntegralsOfMotionAxisymFudge,
     :176-195) and the limits and root brackets of nodeLimitsSetup (ends: as there). */
 static __device__ void nodePrepare(const MultipoleView& M, const double* pc, double Phi, double fd,
-    FudgeRecord& rec, double* act, FudgeEnds* ends = nullptr)
+    FudgeRecord& rec, double* act, FudgeEnds* ends)
 {
     const double R = pc[0], z = pc[1], phi = pc[2], vR = pc[3], vz = pc[4], vphi = pc[5];
     if(fd <= 0) fd = fmax(R, 1.) * 1e-4;
@@ -281,9 +277,7 @@ static __device__ void nodePrepare(const MultipoleView& M, const double* pc, dou
     fnc.M = &M;
     fnc.lambda = lambda;
     fnc.nu = absnu * signz;
-    fnc.phi = 0;                    // axisymmetric potential: its evaluators never read the azimuth
     fnc.D2 = D2;
-    fnc.bad = 0;
     double Phi0;
     CylDerivs g; CylHess h;
     evalMultipoleCylCall<1, EVAL_AXI>(M, sqrt(lambda - D2), 0, 0, &Phi0, &g, &h);

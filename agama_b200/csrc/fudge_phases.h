@@ -24,7 +24,7 @@ void launchNodePrepare(bool finder, const MultipoleView& M, const FudgeTables& F
 /// phase 2: the root searches of the integration limits, drained by a persistent grid from a
 /// device work counter (8 bytes, zeroed here on the stream); with pred (n x 3 predictions) the
 /// searches start on the predicted brackets; stats (4 counters, may be null) accumulates
-/// searches, narrowed searches, fallbacks to the plain bracket and iterations; ends (may be null):
+/// searches, narrowed searches, fallbacks to the plain bracket and iterations; ends:
 /// F and F' at the ends of each record's plain brackets, which the plain searches take instead of
 /// evaluating them again; nodes: F to the bits of the node form of the splines (records whose angles follow)
 void launchFudgeRoots(const MultipoleView& M, long n, FudgeRecord* rec, const FudgeEnds* ends, int* iters,

@@ -35,30 +35,28 @@ enum RootForm { ROOT_CELLS, ROOT_SEGMENTS, ROOT_NODES };
 /// what a lane does next with its search
 enum { LANE_IDLE = 0, LANE_PROPOSE = 1, LANE_EVAL = 2, LANE_VERIFY = 3 };
 
-/** Set up a plain search on its bracket [lo, hi] with F and F' at the ends taken from phase 1
-    (e may be null: the ends are then evaluated by the search): lambda_pos (shared by the lambda
-    brackets), Delta^2 and |nu|; the far end of lambda_max (s = 1, lambda = inf) needs no
+/** Set up a plain search on its bracket [lo, hi] with F and F' at the ends taken from phase 1:
+    lambda_pos (shared by the lambda brackets), Delta^2 and |nu|; the far end of lambda_max (s = 1, lambda = inf) needs no
     evaluation either (limitRootEval's values there).  Returns LANE_IDLE when the search has
     finished at once (no sign change, or a root at an end), LANE_PROPOSE when both ends are known
     and the first iterate is due from RootSearch::propose, LANE_EVAL when *x is an end to evaluate. */
 template<class A>
-__device__ __forceinline__ int setupPlain(RootSearchOf<A>& s, int kind, const FudgeEnds* e, double lo, double hi,
+__device__ __forceinline__ int setupPlain(RootSearchOf<A>& s, int kind, const FudgeEnds& e, double lo, double hi,
     double tol, double u0, double D2, double E, double* x)
 {
-    if(!e) { *x = s.startAbs(lo, hi, tol); return LANE_EVAL; }
     if(kind == ROOT_NU_MAX) {
-        if(hi == D2) return s.setupKnownEnds(lo, hi, tol, e->fNu, e->dfNu, e->fD2, e->dfD2) ? LANE_IDLE : LANE_PROPOSE;
+        if(hi == D2) return s.setupKnownEnds(lo, hi, tol, e.fNu, e.dfNu, e.fD2, e.dfD2) ? LANE_IDLE : LANE_PROPOSE;
         *x = s.startAbs(lo, hi, tol);
-        s.take(e->fNu, e->dfNu, x);         // the lower end known; the upper one is evaluated next
+        s.take(e.fNu, e.dfNu, x);         // the lower end known; the upper one is evaluated next
         return LANE_EVAL;
     }
     if(kind == ROOT_LAMBDA_MIN) {
-        if(lo == D2) return s.setupKnownEnds(lo, hi, tol, e->fD2, e->dfD2, e->fPos, e->dfPos) ? LANE_IDLE : LANE_PROPOSE;
-        *x = s.startKnownUpper(lo, hi, tol, e->fPos, e->dfPos);
+        if(lo == D2) return s.setupKnownEnds(lo, hi, tol, e.fD2, e.dfD2, e.fPos, e.dfPos) ? LANE_IDLE : LANE_PROPOSE;
+        *x = s.startKnownUpper(lo, hi, tol, e.fPos, e.dfPos);
         return LANE_EVAL;
     }
-    const double fa = A::quotient(e->fPos, pow2(u0)),
-        da = A::quotient(e->dfPos - A::quotient(2 * e->fPos, u0), pow2(u0)) * u0;
+    const double fa = A::quotient(e.fPos, pow2(u0)),
+        da = A::quotient(e.dfPos - A::quotient(2 * e.fPos, u0), pow2(u0)) * u0;
     return s.setupKnownEnds(lo, hi, tol, fa, da, E, NAN) ? LANE_IDLE : LANE_PROPOSE;
 }
 
@@ -146,7 +144,7 @@ __global__ void __launch_bounds__(ROOT_BLOCK, FORM != ROOT_CELLS || LEARNED ? 4 
         seeded = false;
         fresh = false;
         if(STATS) nFallback++;
-        mode = setupPlain(s, kind, ends ? ends + point : nullptr, lo, hi, fabs(lo - hi) * FUDGE_ACCURACY_RANGE,
+        mode = setupPlain(s, kind, ends[point], lo, hi, fabs(lo - hi) * FUDGE_ACCURACY_RANGE,
                           u0, fnc.D2, fnc.E, &x);
         if(mode == LANE_IDLE) storePlainLimit(rec[point], kind, s, u0);
     };
@@ -202,7 +200,7 @@ __global__ void __launch_bounds__(ROOT_BLOCK, FORM != ROOT_CELLS || LEARNED ? 4 
                         const double hi = kind == ROOT_NU_MAX ? r.nuUpper : kind == ROOT_LAMBDA_MIN ? r.lambdaPos : 1;
                         const double tol = fabs(lo - hi) * FUDGE_ACCURACY_RANGE;
                         seeded = false;
-                        mode = setupPlain(s, kind, ends ? ends + i : nullptr, lo, hi, tol, u0, r.D2, r.E, &x);
+                        mode = setupPlain(s, kind, ends[i], lo, hi, tol, u0, r.D2, r.E, &x);
                         fresh = mode == LANE_PROPOSE;
                         if(mode == LANE_IDLE)       // no sign change or a root at an end
                             storePlainLimit(rec[i], kind, s, u0);
