@@ -81,7 +81,8 @@ const GLRules& glRulesForCurrentDevice()
 }
 
 constexpr int PREPARE_BLOCK = 128;
-constexpr long POINTS_PER_PASS = 1L << 20;     // records of one pass: 128 MB of scratch
+constexpr long POINTS_PER_PASS = 1L << 20;     // 176 MiB of records and bracket ends a pass,
+                                                // 152 MiB more with angles or frequencies
 
 /// Phase 1, one point per thread: cylindrical coordinates, potential, focal distance (FINDER:
 /// from the finder's table; otherwise fd[i], or fd0 if fd is null), integrals of motion, the

@@ -145,8 +145,9 @@ __device__ __forceinline__ void powerLawAxi(const PowerLawView& A, double rsq, d
     psi (tau_spline = tan(psi / 2)), dx/dtau = 1 / (2 r^2) and dpsi/dtau = K / (2 r^2 sqrt(|tau - D2| tau)),
     K = -sqrt(nu (D2 - nu)) or +sqrt(lambda (lambda - D2)), i.e. -+ D2 c1 c2, with the reciprocal
     roots that R and z are formed from.  One evaluation takes three reciprocal square roots, one
-    reciprocal, a logarithm and an exponential beside the cell (before: three square roots and five
-    to seven divisions, and the gradient's transformation). */
+    reciprocal and a logarithm beside the cell, and with log scaling a second reciprocal and an
+    exponential (before: three square roots and five to seven divisions, and the gradient's
+    transformation). */
 struct FudgeBranch {
     double E, I, L2h, D2;       // I: I3 - fnu (lambda branch) or I3 - flambda; L2h = Lz^2 / 2
     double mo, ro, c1, c2;      // tau - mo multiplies Phi; r^2 = (tau - D2 or tau) + ro

@@ -1,6 +1,6 @@
 // Phase 2 of the Staeckel-fudge actions: the root searches of the integration limits.  In its
-// own compilation unit so that its register budget does not constrain the other phases (the
-// potential evaluator is a non-inlined function compiled once per unit).
+// own compilation unit so that its register budget does not constrain the other phases (what the
+// kernels for potentials without cells call out of line is compiled once per unit).
 #include "runtime.h"
 #include "fudge_nodes.cuh"
 #include "fudge_phases.h"

@@ -1,18 +1,20 @@
 // Device evaluation of the Multipole potential from the coefficients of its spline cells.
 //
 // A cell of a 2-D quintic spline is a polynomial of degree 5 in each of the two positions within
-// the cell, s = (ln r - its lower node) / width and t = (tau - the anchor node) / width.  The node form (multipole_eval.cuh) gathers the 4 x 9 node values of the cell
-// and forms the Hermite basis, six segments in one direction and up to three in the other at every
-// point: ~180 FP64 instructions for value and gradient, with all 36 values and twelve or more
-// intermediates live.  Here the same polynomial is a Horner sum over its 36 monomial coefficients
-// (nine 32-byte loads of one contiguous run): 35 multiply-adds for the value, 75 with
-// the gradient, six independent row sums at a time and only the running sums live, which is what
-// lets the kernels keep more warps on an SM.  Both forms are the same polynomial; their results
-// differ by rounding (the cells' coefficients are formed from the same node data).
+// the cell, s = (ln r - its lower node) / width and t = (tau - the anchor node) / width.  The node
+// form (multipole_eval.cuh) gathers the 4 x 9 node values of the cell and forms the Hermite basis, six
+// segments in one direction and up to three in the other at every point: ~180 FP64 instructions for
+// value and gradient, with all 36 values and twelve or more intermediates live.  Here the same
+// polynomial is a Horner sum over its 36 monomial coefficients (nine 32-byte loads of one contiguous
+// run): 35 multiply-adds for the value, 68 with the gradient, two rows of six at a time and only the
+// running sums live, which is what lets the kernels keep more warps on an SM.  Both forms are the
+// same polynomial; their results differ by rounding (the cells' coefficients are formed from the same
+// node data).
 //
-// The node form stays for callers whose results must not move in the last bits: orbits (chaotic
-// ones amplify a rounding difference without bound) and the construction of the action finder
-// (its grids come from differences of second derivatives).
+// Callers whose results must not move in the last bits have the node form's arithmetic: orbits (chaotic
+// ones amplify a rounding difference without bound) and angles from the segments of the same cells
+// (multipole_force.cuh), the construction of the action finder (its grids come from differences of second
+// derivatives) from the node form itself.
 #pragma once
 #include "multipole_eval.cuh"
 
