@@ -11,9 +11,14 @@ thread_local std::string g_error;
 /// logarithms and powers of the expansions, and the cells for their loads, so more warps are worth some
 /// spilled registers.  Potential alone at 6 / 8 blocks: 54.0 / 51.5 us inside the grid, 99 / 88 beyond it (1e6 points,
 /// disk potential); value and gradient at 5 / 6: 58.0 / 56.0, 123 / 115; with the Hessian at 3 / 4: 76 / 73, 236 / 199.
-/// Potentials without cells keep the compiler's own choice (96 to 228 registers; 1e6 points of one with 17
-/// harmonics: 436 us, 461 at 6 blocks, 517 at one).
-constexpr int minBlocks(int nq, int kind) { return kind == EVAL_GENERAL ? 0 : nq == 1 ? 8 : nq == 3 ? 6 : 4; }
+/// Potentials without cells take the compiler's own choice (96 and 166 registers; 1e6 points of one with 17
+/// harmonics, potential alone: 436 us, 461 at 6 blocks, 517 at one) but for value and gradient, at 4 blocks
+/// (4e5 points at its choice of 164 registers / 5 / 4 blocks: 17 harmonics inside the grid 270 / 266 / 250, inside and beyond it
+/// 1205 / 967 / 1017, a lopsided l <= 2 potential 226 / 232 / 216).
+constexpr int minBlocks(int nq, int kind)
+{
+    return kind == EVAL_GENERAL ? (nq == 3 ? 4 : 0) : nq == 1 ? 8 : nq == 3 ? 6 : 4;
+}
 
 /// One point per thread; 128 threads per block.  NQ = 1 (potential), 3 (+gradient), 6 (+Hessian);
 /// KIND = spline evaluator matching the potential (EvalKind).  Bound by the L1: each lane reads its own
